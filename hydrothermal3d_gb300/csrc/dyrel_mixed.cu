@@ -2,6 +2,7 @@
 #include <cuda.h>
 #include <algorithm>
 #include <cstddef>
+#include <iterator>
 #include <mutex>
 
 #include "dyrel_common.cuh"
@@ -685,6 +686,8 @@ __global__ void __launch_bounds__(TB_LANES* TB_Y, TB_Y <= 8 ? 2 : 1) k_mixed_inn
 }
 constexpr size_t kTbSmem = 128 + sizeof(TbStage) * TB_STAGES + sizeof(float) * 2 * kTbRd + 8 * TB_STAGES;
 
+#include "dyrel_resident.cuh"
+
 // cuTensorMapEncodeTiled, fetched from the driver at run time (no libcuda link)
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -1109,6 +1112,32 @@ int ht3d_dyrel_solve_mixed(ht3d_ctx* ctx, double* X, const double* R, const doub
         derr = (int*)ht3d_scratch(ctx, SLOT_AUX0, sizeof(int) * 16);
         HT3D_CUDA(cudaMemsetAsync(derr, 0, sizeof(int), ctx->stream));
     }
+    // runs of inner iterations in one launch, where the grid fits the chip and
+    // the caller left the iteration to the library (a batched tile shape or a
+    // temporal setting of their own means the kernels that these select)
+    const bool may_reside = ctx->mixed_temporal == 1 && !ctx->ens_tile && !ctx->ens_block && !ctx->res_off;
+    const ResPlan plan = may_reside && !pairs ? res_plan(P, ctx->num_sms) : ResPlan();
+    bool resident = plan.bz > 0;
+    if (resident) {
+        derr = (int*)ht3d_scratch(ctx, SLOT_AUX0, sizeof(int) * 16);
+        HT3D_CUDA(cudaMemsetAsync(derr, 0, sizeof(int), ctx->stream));
+    }
+    // the run iter .. run_end (at least two iterations) in one launch
+    auto run_resident = [&](int iter, int run_end, const MixScal& s32, bool prev0, int cur, int prv) {
+        ResLaunch L;
+        L.n = 1;
+        L.iters = run_end - iter + 1;
+        L.prev0 = prev0 ? 1 : 0;
+        L.skip = ctx->wait_test;
+        L.limit = ctx->wait_test > 0 ? 1u << 12 : kResWaitLimit;
+        ctx->wait_test = 0;
+        L.err = derr;
+        L.block0[0] = 0;
+        L.block0[1] = plan.ctas();
+        u64* x = res_exchange(ctx, res_words(plan), L.iters, L.tag);
+        L.rec[0] = res_member(plan, P, Dbuf[cur], Dbuf[prv], Rin, kx32, ky32, kz32, Dbuf[cur], Dbuf[prv], s32, bch, x);
+        return res_launch(ctx, plan.bz, L, plan.T, res_smem(plan.bz, plan.nq, plan.by));
+    };
     InnerTimer timer(ctx);
     double* xcur = X;
     double* xnxt = X2;
@@ -1155,6 +1184,19 @@ int ht3d_dyrel_solve_mixed(ht3d_ctx* ctx, double* X, const double* R, const doub
             while (run_end < nmax && !is_fp64(run_end + 1)) ++run_end;
             const int pair_end = run_end == nmax ? run_end - 1 : run_end;
             const int left = pair_end - iter + 1;
+            // (an iteration that has to leave F goes by itself)
+            const int res_end = run_end - (run_end == nmax || is_check(run_end + 1, prm->nitout) ? 1 : 0);
+            if (resident && res_end > iter && dtau_prev == sc.dtau) {
+                resident = run_resident(iter, res_end, s32, prev0, cur, prv);
+                ctx->res_off = !resident;
+                if (resident) {
+                    timer.count(res_end - iter + 1);
+                    prev0 = false;
+                    it_done = iter = res_end;
+                    last_fp64 = last_chk = false;
+                    continue;
+                }
+            }
             // a pass starts only on a steady iteration (Dprev stored, mom = h1)
             if (pairs && !prev0 && dtau_prev == sc.dtau && left >= 2 && left % 2 == 0) {
                 const bool storef2 = iter + 1 == nmax || is_check(iter + 2, prm->nitout);
@@ -1211,7 +1253,7 @@ int ht3d_dyrel_solve_mixed(ht3d_ctx* ctx, double* X, const double* R, const doub
     }
     HT3D_LAUNCH(ctx, k_unpack_f0, gc, b2, 0, F0, Dbuf[cur], prev0 ? nullptr : Dbuf[prv], (float)dtau_prev, P);
     if (!last_chk) HT3D_LAUNCH(ctx, k_unpack, gc, b2, 0, F, Fs, P);
-    if (derr) {  // a bounded wait of k_mixed_inner2 gave up
+    if (derr) {  // a bounded wait of k_mixed_inner2 or k_mixed_resident gave up
         int herr = 0;
         HT3D_CUDA(cudaMemcpyAsync(&herr, derr, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
         HT3D_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1530,6 +1572,75 @@ void ht3d_ensemble_solve_mixed(ht3d_ctx* ctx, EnsSolveInst* in, int n) {
         }
     bool graphs = ctx->ens_graphs != 0;
 
+    // ---- runs of inner iterations in one launch per wave of members that fit
+    // the chip together (unless the caller chose a tile shape)
+    std::vector<ResPlan> plans(n);
+    bool resident = !ctx->ens_tile && !ctx->ens_block && !ctx->res_off && ctx->mixed_temporal == 1;
+    for (int q : order) {
+        if (resident) plans[q] = res_plan_full(H[q].P, ctx->num_sms);
+        resident = resident && plans[q].bz;
+    }
+    int* derr = nullptr;
+    if (resident) {
+        tuning = false;
+        if (cfg < 0) cfg = 1;  // for the iterations that go by themselves
+        derr = (int*)ht3d_scratch(ctx, SLOT_AUX0, sizeof(int) * 16);
+        HT3D_CUDA(cudaMemsetAsync(derr, 0, sizeof(int), ctx->stream));
+    }
+    // iterations iter .. res_end of every active member, a wave after the other
+    auto run_resident = [&](int iter, int res_end, int parity, int prev0) {
+        const int iters = res_end - iter + 1, to = (parity + iters) & 1;
+        std::vector<int> left;
+        for (int q : order)
+            if (H[q].active) left.push_back(q);
+        // equal columns together, the largest grids first, then whatever still fits
+        std::stable_sort(left.begin(), left.end(), [&](int a, int b) {
+            return plans[a].bz != plans[b].bz ? plans[a].bz > plans[b].bz : plans[a].ctas() > plans[b].ctas();
+        });
+        bool first = true;
+        while (!left.empty()) {
+            ResLaunch L;
+            L.n = 0;
+            L.iters = iters;
+            L.prev0 = prev0;
+            L.skip = 0;
+            L.limit = kResWaitLimit;
+            L.err = derr;
+            L.block0[0] = 0;
+            const int bz = plans[left[0]].bz, cap = ctx->num_sms;
+            std::vector<int> wave, rest;
+            size_t words = 0, smem = 0;
+            int threads = 0;
+            for (int q : left) {
+                const ResPlan& p = plans[q];
+                if (p.bz != bz || L.n == kResMaxPerLaunch || L.block0[L.n] + p.ctas() > cap) {
+                    rest.push_back(q);
+                    continue;
+                }
+                wave.push_back(q);
+                L.block0[L.n + 1] = L.block0[L.n] + p.ctas();
+                ++L.n;
+                words += res_words(p);
+                smem = std::max(smem, res_smem(p.bz, p.nq, p.by));
+                threads = std::max(threads, p.T);
+            }
+            u64* x = res_exchange(ctx, words, iters, L.tag);
+            for (int m = 0; m < L.n; ++m) {
+                EnsHost& h = H[wave[m]];
+                L.rec[m] = res_member(plans[wave[m]], h.P, h.f32[parity], h.f32[parity ^ 1], h.f32[3], h.f32[4], h.f32[5],
+                                      h.f32[6], h.f32[to], h.f32[to ^ 1], mix_scal(h.sc, h.dtau_prev), h.bch, x);
+                x += res_words(plans[wave[m]]);
+            }
+            if (!res_launch(ctx, bz, L, threads, smem)) {
+                if (first) return false;
+                throw ht3d_error(HT3D_ERR_CUDA, "cooperative launch refused between the waves of an ensemble");
+            }
+            first = false;
+            left.swap(rest);
+        }
+        return true;
+    };
+
     const int refresh_every = ctx->mixed_refresh;
     auto is_fp64 = [&](int it) { return is_check(it, nitout) || (refresh_every > 0 && it % refresh_every == 0); };
     auto is_storef = [&](int it) { return !is_fp64(it) && (it == nitmax || is_check(it + 1, nitout)); };
@@ -1571,54 +1682,68 @@ void ht3d_ensemble_solve_mixed(ht3d_ctx* ctx, EnsSolveInst* in, int n) {
             timer.begin();
             const bool storef = is_storef(iter);
             int window = 1;
-            if (!storef && !tuning && graphs && !prev0) {
-                window = 0;
-                while (window < kEnsGraphIters && iter + window <= nitmax && !is_fp64(iter + window) &&
-                       !is_storef(iter + window))
-                    ++window;
-                if (window == kEnsGraphIters) {
-                    graphs = ens_capture(ctx, graph_sig(version, cfg), cfg, groups[cfg]);
-                    if (!graphs) window = 1;
-                } else {
-                    window = 1;
-                }
+            int res_end = iter;  // the run's last iteration that does not leave F
+            while (resident && res_end < nitmax && !is_fp64(res_end + 1) && !is_storef(res_end + 1)) ++res_end;
+            bool steady = res_end > iter && !storef;
+            for (int q = 0; q < n && steady; ++q) steady = !H[q].active || H[q].dtau_prev == H[q].sc.dtau;
+            if (steady && !run_resident(iter, res_end, parity, prev0)) {  // one launch per iteration from here on
+                ctx->res_off = true;
+                resident = false;
+                steady = false;
             }
-            if (window == kEnsGraphIters) {
-                HT3D_CUDA(cudaGraphLaunch(ctx->ens_graph[parity], ctx->stream));
-                ctx->launches += (unsigned long long)kEnsGraphIters * groups[cfg].size();
-                for (int g = 0; g < kEnsGraphIters; ++g) timer.count();
+            if (steady) {
+                window = res_end - iter + 1;
+                timer.count(window);
             } else {
-                int c = tuning ? 1 : cfg;
-                const bool timed = tuning && !storef;
-                if (timed) {
-                    c = tune_n % kEnsNCfg;
-                    HT3D_CUDA(cudaEventRecord(ctx->tune_events[2 * tune_n], ctx->stream));
+                if (!storef && !tuning && graphs && !prev0) {
+                    window = 0;
+                    while (window < kEnsGraphIters && iter + window <= nitmax && !is_fp64(iter + window) &&
+                           !is_storef(iter + window))
+                        ++window;
+                    if (window == kEnsGraphIters) {
+                        graphs = ens_capture(ctx, graph_sig(version, cfg), cfg, groups[cfg]);
+                        if (!graphs) window = 1;
+                    } else {
+                        window = 1;
+                    }
                 }
-                const int nl = storef ? ens_launch_all<true>(ctx->stream, c, groups[c], parity, prev0)
-                                      : ens_launch_all<false>(ctx->stream, c, groups[c], parity, prev0);
-                ctx->launches += nl;
-                timer.count();
-                if (timed) {
-                    HT3D_CUDA(cudaEventRecord(ctx->tune_events[2 * tune_n + 1], ctx->stream));
-                    if (++tune_n == kEnsNCfg * kEnsTuneRounds) {
-                        HT3D_CUDA(cudaEventSynchronize(ctx->tune_events[2 * tune_n - 1]));
-                        float best = 0.f;
-                        for (int cc = 0; cc < kEnsNCfg; ++cc) {
-                            float sum = 0.f;
-                            for (int r = 0; r < kEnsTuneRounds; ++r) {
-                                float ms = 0.f;
-                                const int t = r * kEnsNCfg + cc;
-                                HT3D_CUDA(cudaEventElapsedTime(&ms, ctx->tune_events[2 * t], ctx->tune_events[2 * t + 1]));
-                                sum += ms;
+                if (window == kEnsGraphIters) {
+                    HT3D_CUDA(cudaGraphLaunch(ctx->ens_graph[parity], ctx->stream));
+                    ctx->launches += (unsigned long long)kEnsGraphIters * groups[cfg].size();
+                    for (int g = 0; g < kEnsGraphIters; ++g) timer.count();
+                } else {
+                    int c = tuning ? 1 : cfg;
+                    const bool timed = tuning && !storef;
+                    if (timed) {
+                        c = tune_n % kEnsNCfg;
+                        HT3D_CUDA(cudaEventRecord(ctx->tune_events[2 * tune_n], ctx->stream));
+                    }
+                    const int nl = storef ? ens_launch_all<true>(ctx->stream, c, groups[c], parity, prev0)
+                                          : ens_launch_all<false>(ctx->stream, c, groups[c], parity, prev0);
+                    ctx->launches += nl;
+                    timer.count();
+                    if (timed) {
+                        HT3D_CUDA(cudaEventRecord(ctx->tune_events[2 * tune_n + 1], ctx->stream));
+                        if (++tune_n == kEnsNCfg * kEnsTuneRounds) {
+                            HT3D_CUDA(cudaEventSynchronize(ctx->tune_events[2 * tune_n - 1]));
+                            float best = 0.f;
+                            for (int cc = 0; cc < kEnsNCfg; ++cc) {
+                                float sum = 0.f;
+                                for (int r = 0; r < kEnsTuneRounds; ++r) {
+                                    float ms = 0.f;
+                                    const int t = r * kEnsNCfg + cc;
+                                    HT3D_CUDA(cudaEventElapsedTime(&ms, ctx->tune_events[2 * t], ctx->tune_events[2 * t + 1]));
+                                    sum += ms;
+                                }
+                                if (cc == 0 || sum < best) {
+                                    best = sum;
+                                    cfg = cc;
+                                }
                             }
-                            if (cc == 0 || sum < best) {
-                                best = sum;
-                                cfg = cc;
-                            }
+                            tuning = false;
+                            ctx->ens_tune_key = shape;
+                            ctx->ens_tune_cfg = cfg + 1;
                         }
-                        tuning = false;
-                        ctx->ens_tune_key = shape;
-                        ctx->ens_tune_cfg = cfg + 1;
                     }
                 }
             }
@@ -1676,6 +1801,16 @@ void ht3d_ensemble_solve_mixed(ht3d_ctx* ctx, EnsSolveInst* in, int n) {
         if (!h.last_chk) HT3D_LAUNCH(ctx, k_unpack, gc, b2, 0, I.F, h.f32[2], h.P);
         h.C.fill(I.st, h.S, h.it_done);
         in[q].status = h.C.status;
+    }
+    if (derr) {  // a bounded wait of k_mixed_resident gave up: no member's fields are to be trusted
+        int herr = 0;
+        HT3D_CUDA(cudaMemcpyAsync(&herr, derr, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        HT3D_CUDA(cudaStreamSynchronize(ctx->stream));
+        for (int q = 0; q < n && herr; ++q)
+            if (H[q].used) {
+                in[q].status = herr;
+                if (in[q].st) in[q].st->status = herr;
+            }
     }
     timer.collect();
 }

@@ -33,6 +33,7 @@ enum ScratchSlot {
     SLOT_AUX0, SLOT_AUX1, SLOT_AUX2, SLOT_AUX3,
     SLOT_ENS_SOLVE,     // batched solve: per-instance FP64 and padded FP32 fields
     SLOT_ENS_TAB,       // batched solve: per-instance check results
+    SLOT_RES,           // resident iterations: face words of the blocks
     SLOT_ENS_STEP,      // ensemble step: per-instance residual, flux and conductivity fields
     SLOT_COUNT
 };
@@ -62,6 +63,8 @@ struct ht3d_ctx {
     cudaGraphExec_t ens_graph[2] = {nullptr, nullptr};  // windows starting on parity 0 / 1
     void* h_ens = nullptr;                // pinned staging (instance records, results)
     size_t h_ens_bytes = 0;
+    unsigned res_tag = 0;                 // iterations numbered so far by the resident kernel (this context)
+    bool res_off = false;                 // the device refused a cooperative launch: iterate one launch at a time
     int num_sms = 152;
     unsigned long long launches = 0;
     std::string last_error;
