@@ -1,0 +1,62 @@
+// FP64 quotients in few operations.
+//
+// GB300 issues an FP64 operation for one warp every 64 cycles per scheduler (2
+// results per clock and SM), and an IEEE division costs nine or ten of them.
+// The quotients here take an approximate reciprocal y of the divisor (refined by
+// Newton's iteration, or rounded on the host for a divisor that a launch shares)
+// and correct a y once by its exact remainder, r = a - b q with one fma, q' =
+// fma(r, y, q) (P. Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990): q' is the
+// correctly rounded quotient unless a / b lies within about 2^-51 ulp of the
+// middle between two doubles, which one pair of operands in 10^15 does; there
+// it may be the other neighbour.  Operands outside the range in which nothing
+// over- or underflows on the way (zero, infinite and NaN among them) are
+// divided by the operator.
+#pragma once
+#include <cuda_runtime.h>
+
+// exponent test of the fast path: 2^-400 <= |x| < 2^400 (integer operations)
+__device__ __forceinline__ bool mid_range(double x) {
+    return ((unsigned)__double2hiint(x) & 0x7fffffffu) - 0x26f00000u < 0x32000000u;
+}
+// ... or 0, as a dividend
+__device__ __forceinline__ bool mid_range0(double x) {
+    return mid_range(x) || (((unsigned)__double2hiint(x) & 0x7fffffffu) | (unsigned)__double2loint(x)) == 0u;
+}
+// 1/b to about an ulp: the hardware's approximation (20 bits or more), refined
+// to third order: y (1 + e + e^2), e = 1 - b y
+__device__ __forceinline__ double rcp_newton(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    const double e = __fma_rn(-b, y, 1.0);
+    return __fma_rn(y, __fma_rn(e, e, e), y);
+}
+// a / b from y = 1/b to an ulp or so; a, b and a/b in the middle of the range
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+    const double q = __dmul_rn(a, y);
+    return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+// a / b for any operands
+__device__ __forceinline__ double div_any(double a, double b) {
+    if (mid_range0(a) && mid_range(b)) return div_by(a, b, rcp_newton(b));
+    return __ddiv_rn(a, b);
+}
+// a / b where y = 1/b is at hand
+__device__ __forceinline__ double div_known(double a, double b, double y) {
+    if (mid_range0(a) && mid_range(b)) return div_by(a, b, y);
+    return __ddiv_rn(a, b);
+}
+// A divisor that a launch shares, with its reciprocal rounded on the host.
+struct Divisor {
+    double b, y;
+    Divisor() = default;
+    __host__ explicit Divisor(double d) : b(d), y(1.0 / d) {}
+};
+__device__ __forceinline__ double operator/(double a, const Divisor& d) { return div_known(a, d.b, d.y); }
+
+// v / 3, correctly rounded (but for subnormal results): 1/3 as the sum of two
+// doubles; v/3 is at least a sixth of an ulp away from any middle between two
+// doubles, and the sum errs by 2^-53 ulp.
+__device__ __forceinline__ double third(double v) {
+    return __fma_rn(v, 0x1.5555555555555p-2, __dmul_rn(v, 0x1.5555555555555p-56));
+}

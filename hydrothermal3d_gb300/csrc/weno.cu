@@ -44,18 +44,23 @@ __global__ void __launch_bounds__(256) k_weno_stage(const double* __restrict__ s
     else if (AXIS == 1) { vl = ix3(i, j, k, nx, ny + 1); vs = nx; }
     else { vl = ix3(i, j, k, nx, ny); vs = (long long)nx * ny; }
     const double a = V[vl], b = V[vl + vs];
-    const double Vm = a < 0.0 ? a : 0.0;
-    const double Vp = b >= 0.0 ? b : 0.0;
+    const double Vm = neg_part(a), Vp = pos_part(b);
     double rhs;
     if (PREC == 0) {
-        // x[o] holds X[I+o-3]
-        const double m1 = h * (x[1] - x[0]), m2 = h * (x[2] - x[1]), m3 = h * (x[3] - x[2]), m4 = h * (x[4] - x[3]);
-        const double m5 = QUIRK ? h * (x[5] - x[2]) : h * (x[5] - x[4]);
-        const double dFm = upwind_active(Vp) ? weno5_ref(m1, m2, m3, m4, m5) : 0.0;
-        const double p1 = h * (x[6] - x[5]), p2 = h * (x[5] - x[4]), p3 = h * (x[4] - x[3]), p4 = h * (x[3] - x[2]);
-        const double p5 = h * (x[2] - x[1]);
-        const double dFp = upwind_active(Vm) ? weno5_ref(p1, p2, p3, p4, p5) : 0.0;
-        rhs = Vp * dFm + Vm * dFp;
+        // x[o] holds X[I+o-3].  A point has one inflow side almost always: its
+        // lane selects that side's differences, so a warp whose flow changes sign
+        // evaluates one derivative per lane and not both for all (127^3 sweep:
+        // 4.38 -> 3.40 ms).
+        double d[6];
+#pragma unroll
+        for (int o = 0; o < 6; ++o) d[o] = h * (x[o + 1] - x[o]);
+        const double m5 = QUIRK ? h * (x[5] - x[2]) : d[4];
+        const bool minus = upwind_active(Vp), plus = upwind_active(Vm);
+        rhs = 0.0;  // Vp dF- + Vm dF+, a product with a zero factor left out
+        if (minus || plus)
+            rhs = (minus ? Vp : Vm) * weno5_ref(minus ? d[0] : d[5], minus ? d[1] : d[4], minus ? d[2] : d[3],
+                                                minus ? d[3] : d[2], minus ? m5 : d[1]);
+        if (minus && plus) rhs += Vm * weno5_ref(d[5], d[4], d[3], d[2], d[1]);
     } else {
         // FP64 differences e[o] = X[I+o-2] - X[I+o-3]; FP32 copies scaled by h
         // for the smoothness indicators (weno5_mixed)
@@ -77,7 +82,7 @@ __global__ void __launch_bounds__(256) k_weno_stage(const double* __restrict__ s
     }
     const double t = x[3] - dt * rhs;
     if (STAGE == 1) dst[e] = t;
-    else dst[e] = 0.5 * t + 0.5 * T0[e];
+    else dst[e] = PREC == 0 ? __fma_rn(0.5, t, 0.5 * T0[e]) : 0.5 * t + 0.5 * T0[e];  // 0.5 t is exact
 }
 
 // ------------------------------------------------------- granular drop-ins

@@ -203,20 +203,6 @@ struct WenoStreamWindow {
 template <int QUIRK> struct StreamOf { using type = WenoStreamWindow<QUIRK>; };
 template <> struct StreamOf<0> { using type = WenoStreamShared; };
 
-// The upwind factors of an FP64 face velocity, v < 0 ? v : 0 and
-// v >= 0 ? v : 0 (NaN gives 0), from the bit pattern: integer operations
-// instead of two compares on the FP64 pipe.
-__device__ __forceinline__ double neg_part(double v) {
-    const long long b = __double_as_longlong(v);
-    const unsigned long long m = (unsigned long long)b & 0x7fffffffffffffffULL;
-    return (b < 0 && m != 0 && m <= 0x7ff0000000000000ULL) ? v : 0.0;
-}
-__device__ __forceinline__ double pos_part(double v) {
-    const long long b = __double_as_longlong(v);
-    const unsigned long long m = (unsigned long long)b & 0x7fffffffffffffffULL;
-    return (m <= 0x7ff0000000000000ULL && (b >= 0 || m == 0)) ? v : 0.0;
-}
-
 // Mixed-precision form of the face-shared stream (the WENO5 stage of the
 // mixed solver, weno5_mixed's split): T, the one-sided differences e (here
 // unscaled, FP64), their second differences a and third differences g, and
