@@ -2,7 +2,7 @@
 // rounds exactly like the reference's separate kernels (no FMA contraction,
 // F divided by PC), so the solver differs from the reference only through the
 // summation order of its norm and Rayleigh-quotient reductions.
-#include "dyrel_common.cuh"
+#include "dyrel_f64.cuh"
 
 int ht3d_dyrel_solve_fp64(ht3d_ctx* ctx, double* X, const double* R, const double* kx, const double* ky,
                           const double* kz, double cX, double dx, double dy, double dz, const int* bc_type6,
@@ -14,6 +14,9 @@ int ht3d_dyrel_solve_fp64(ht3d_ctx* ctx, double* X, const double* R, const doubl
     double* PC = (double*)ht3d_scratch(ctx, SLOT_PC, sizeof(double) * n);
     double* X2 = (double*)ht3d_scratch(ctx, SLOT_X2, sizeof(double) * nex);
     IterLaunch L = iter_launch(ctx, nx, ny, nz);
+    const bool fixed_variant = ctx->dyrel_variant != 0;  // the caller's thread layout
+    const F64Launch L64 = f64_launch(ctx->num_sms, nx, ny, nz);
+    double* iPC = fixed_variant ? nullptr : (double*)ht3d_scratch(ctx, SLOT_G, sizeof(double) * n);
     const long long nsetup = (long long)((nx + 31) / 32) * ((ny + 7) / 8) * nz;
     // per-cell check terms (3n) followed by tree-pass work space
     const long long nwork = 3 * n + 6 * ((n + 1023) / 1024 + 1);
@@ -32,6 +35,7 @@ int ht3d_dyrel_solve_fp64(ht3d_ctx* ctx, double* X, const double* R, const doubl
         const double transient = cX != 0.0 ? 1.0 : 0.0, dt = cX != 0.0 ? 1.0 / cX : 1.0;
         HT3D_LAUNCH(ctx, k_dyrel_setup<0>, g, b, 0, kx, ky, kz, 1.0, transient, dt, dx, dy, dz, nx, ny, nz, PC, parts);
         HT3D_LAUNCH(ctx, (k_reduce_partials<RED_MAX, 1>), 1, 1024, 0, parts, (int)(g.x * g.y * g.z), dres);
+        if (iPC) HT3D_LAUNCH(ctx, k_reciprocal, (unsigned)std::min<long long>((n + 255) / 256, ctx->num_sms * 16LL), 256, 0, iPC, PC, n);
         ht3d_fetch_results(ctx, dres, 1);
     }
     DyrelState S;
@@ -56,7 +60,14 @@ int ht3d_dyrel_solve_fp64(ht3d_ctx* ctx, double* X, const double* R, const doubl
         sc.h1 = S.h1;
         sc.h2 = S.h2;
         sc.dtau = S.dtau;
-        if (chk)
+        if (iPC) {
+            const bool cx = cX != 0.0;
+            const auto kern = chk ? F64Kernel<MODE_CHECK>::get(cx, true, L64.threads)
+                                  : (storef ? F64Kernel<MODE_STOREF>::get(cx, true, L64.threads)
+                                            : F64Kernel<MODE_PLAIN>::get(cx, true, L64.threads));
+            HT3D_LAUNCH(ctx, kern, L64.grid, L64.threads, 0, cur, nxt, R, kx, ky, kz, PC, iPC, F0, F,
+                        DyrelScalT<double>(sc), bc, nx, ny, nz, L64.zchunk, parts);
+        } else if (chk)
             launch_iter<double, MODE_CHECK>(ctx, L, cur, nxt, R, kx, ky, kz, PC, F0, F, sc, bc, nx, ny, nz, parts);
         else if (storef)
             launch_iter<double, MODE_STOREF>(ctx, L, cur, nxt, R, kx, ky, kz, PC, F0, F, sc, bc, nx, ny, nz, parts);
@@ -111,8 +122,41 @@ extern "C" int ht3d_dyrel_iterate(ht3d_ctx* ctx, double* X_ex, const double* R, 
                                   double dz, const int* bc_type6, const double* bc_val6, double h1, double h2,
                                   double dtau, int n_iter, int nx, int ny, int nz) {
     return ht3d_guard(ctx, [&]() {
-        return dyrel_iterate_impl<double>(ctx, X_ex, R, kx, ky, kz, PC, F0, cX, dx, dy, dz, bc_type6, bc_val6, h1,
-                                          h2, dtau, n_iter, nx, ny, nz, SLOT_AUX0);
+        if (ctx->dyrel_variant)
+            return dyrel_iterate_impl<double>(ctx, X_ex, R, kx, ky, kz, PC, F0, cX, dx, dy, dz, bc_type6, bc_val6, h1,
+                                              h2, dtau, n_iter, nx, ny, nz, SLOT_AUX0);
+        ht3d_check_dims(nx, ny, nz, 1);
+        HT3D_REQUIRE(X_ex && R && kx && ky && kz && PC && F0 && bc_type6 && bc_val6, "null argument");
+        HT3D_REQUIRE(n_iter >= 0, "n_iter must be >= 0");
+        const long long n = (long long)nx * ny * nz, nex = (long long)(nx + 2) * (ny + 2) * (nz + 2);
+        BC6<double> bc;
+        for (int f = 0; f < 6; ++f) {
+            HT3D_REQUIRE(bc_type6[f] == HT3D_BC_NEUMANN || bc_type6[f] == HT3D_BC_DIRICHLET, "face BC type must be 0 or 1");
+            bc.dir[f] = bc_type6[f];
+            bc.val2[f] = 2.0 * bc_val6[f];
+        }
+        double* X2 = (double*)ht3d_scratch(ctx, SLOT_AUX0, sizeof(double) * nex);
+        // the reciprocals pay from a few iterations on (3 operations a cell each instead of 6, and 1 division here)
+        double* iPC = nullptr;
+        if (n_iter >= 4) {
+            iPC = (double*)ht3d_scratch(ctx, SLOT_G, sizeof(double) * n);
+            HT3D_LAUNCH(ctx, k_reciprocal, (unsigned)std::min<long long>((n + 255) / 256, ctx->num_sms * 16LL), 256, 0, iPC, PC, n);
+        }
+        const F64Launch L = f64_launch(ctx->num_sms, nx, ny, nz);
+        const DyrelScalT<double> sc(DyrelScal{h1, h2, dtau, cX, 1.0 / dx, 1.0 / dy, 1.0 / dz});
+        const auto kern = F64Kernel<MODE_PLAIN>::get(cX != 0.0, iPC != nullptr, L.threads);
+        double* cur = X_ex;
+        double* nxt = X2;
+        for (int it = 0; it < n_iter; ++it) {
+            HT3D_LAUNCH(ctx, kern, L.grid, L.threads, 0, cur, nxt, R, kx, ky, kz, PC, iPC, F0, (double*)nullptr, sc,
+                        bc, nx, ny, nz, L.zchunk, (double*)nullptr);
+            std::swap(cur, nxt);
+        }
+        if (cur != X_ex) {
+            dim3 b(32, 8, 1), g((nx + 2 + 31) / 32, (ny + 2 + 7) / 8, nz + 2);
+            HT3D_LAUNCH(ctx, k_copy_ex_faces<double>, g, b, 0, X_ex, cur, nx, ny, nz);
+        }
+        return HT3D_OK;
     });
 }
 

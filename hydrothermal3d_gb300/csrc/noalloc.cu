@@ -16,7 +16,7 @@
 #include <mutex>
 #include <utility>
 
-#include "dyrel_common.cuh"
+#include "dyrel_f64.cuh"
 
 namespace {
 
@@ -89,12 +89,15 @@ extern "C" int ht3d_dyrel_iterate_noalloc(double* X_ex, const double* R, const d
     if (s != HT3D_OK) return s;
     cudaStream_t st = (cudaStream_t)stream;
     const DyrelScalT<double> sc(DyrelScal{h1, h2, dtau, cX, 1.0 / dx, 1.0 / dy, 1.0 / dz});
-    const dim3 blk(CX_, CY_, CZ_), grd((nx + CX_ - 1) / CX_, (ny + CY_ - 1) / CY_, (nz + CZ_ - 1) / CZ_);
+    // 152 SMs for the plane chunks (the result does not depend on them)
+    const F64Launch L = f64_launch(152, nx, ny, nz);
+    const auto kern = F64Kernel<MODE_PLAIN>::get(cX != 0.0, false, L.threads);
     double* cur = X_ex;
     double* nxt = scratch;
     for (int it = 0; it < n_iter; ++it) {
-        const cudaError_t e = launch(k_dyrel_cell<double, MODE_PLAIN>, grd, blk, st, cur, nxt, R, kx, ky, kz, PC, F0,
-                                     (double*)nullptr, sc, bc, nx, ny, nz, (double*)nullptr);
+        const cudaError_t e = launch(kern, L.grid, L.threads, st, cur, nxt, R, kx, ky, kz, PC,
+                                     (const double*)nullptr, F0, (double*)nullptr, sc, bc, nx, ny, nz, L.zchunk,
+                                     (double*)nullptr);
         if (e != cudaSuccess) return HT3D_ERR_CUDA;
         std::swap(cur, nxt);
     }
