@@ -9,12 +9,13 @@
 // after row without gaps, and marches through a chunk of planes.  A thread
 // evaluates its cells' west and south fluxes and leaves them in shared memory
 // for the pair to the west and the row to the south; the z flux stays in a
-// register.  What is left are 9 operations for the fluxes (15 in k_dyrel_iter),
+// register.  (Small grids: one cell per thread.)  What is left are 9 operations for the fluxes (15 in k_dyrel_iter),
 // 9 or 11 for their sum, 3 for the quotient (9) and 5 for the update, and one
 // more face at the block's end, at a wall and at a chunk's first plane.
 //
-// us per iteration, k_dyrel_iter and this kernel: 31 x 29 x 33 8.5 -> 6.5, 63^3
-// 31.0 -> 22.9, 95^3 82 -> 62, 127 x 119 x 131 180 -> 133, 255^3 1440 -> 1006.
+// us per iteration, k_dyrel_iter and this kernel: 31 x 29 x 33 8.5 -> 4.9, 63^3
+// 31.0 -> 20.6, 95^3 82 -> 58.5, 127 x 119 x 131 180 -> 131, 255^3 1440 -> 1009.
+// Plain launches begin on a 2 us raster; launch_after saves the wait (63^3: 22.9).
 #pragma once
 #include "dyrel_common.cuh"
 #include "fp64_div.cuh"
@@ -28,8 +29,9 @@ __device__ __forceinline__ double ghost_f64(const BC6<double>& bc, int f, double
     return v;
 }
 
-// CX: cX != 0 (adding 0 * x changes no value).  INV: iPC holds 1 / PC.
-template <int MODE, bool CX, bool INV, int T>
+// CX: cX != 0 (adding 0 * x changes no value).  INV: iPC holds 1 / PC.  NC: cells
+// per thread, neighbours in x.
+template <int MODE, bool CX, bool INV, int T, int NC>
 __global__ void __launch_bounds__(T) k_dyrel_f64(const double* __restrict__ Xin, double* __restrict__ Xout,
                                                 const double* __restrict__ R, const double* __restrict__ kx,
                                                 const double* __restrict__ ky, const double* __restrict__ kz,
@@ -38,131 +40,123 @@ __global__ void __launch_bounds__(T) k_dyrel_f64(const double* __restrict__ Xin,
                                                 BC6<double> bc, int nx, int ny, int nz, int zchunk,
                                                 double* __restrict__ partials) {
     // west flux of the first cell and south fluxes, two planes deep: one barrier per plane
-    __shared__ double west[2][T];
-    __shared__ double2 south[2][T];
-    const int np = (nx + 1) / 2, tid = threadIdx.x;
+    __shared__ double west[2][T], south[2][NC][T];
+    after_previous();
+    const int np = (nx + NC - 1) / NC, tid = threadIdx.x;
     const int t = blockIdx.x * T + tid;
-    const int j = t / np, i = 2 * (t - j * np);
-    const bool row = j < ny, in1 = i + 1 < nx;
+    const int j = t / np, i = NC * (t - j * np);
+    const bool row = j < ny;
     const int k0 = blockIdx.z * zchunk, k1 = min(nz, k0 + zchunk);
     const double h1 = s.h1, h2 = s.h2, dtau = s.dtau, _dx = s._dx, _dy = s._dy, _dz = s._dz;
-    const bool east_here = i + 2 == nx || (tid == T - 1 && i + 2 < nx);  // east face of cell 1: no thread's west face
-    const bool north_here = j == ny - 1 || tid + np >= T;
+    const int nc = min(NC, nx - i);                                          // cells of this thread
+    const bool wall = i + NC == nx;                                          // its last face is the wall
+    const bool east_here = wall || (tid == T - 1 && i + NC < nx);            // that face is no thread's west face
+    const bool north_here = j >= ny - 1 || tid + np >= T;
     const int n1 = nx + 2, pl = n1 * (ny + 2), cpl = nx * ny;
     const int jc = min(j, ny - 1);  // threads past the plane read its last row and store nothing
     int e = (i + 1) + n1 * (jc + 1) + pl * (k0 + 1);
     int c = i + nx * jc + cpl * k0;
     int fx = i + (nx + 1) * (jc + ny * k0), fy = i + nx * (jc + (ny + 1) * k0);
-    const int d1 = in1 ? 1 : 0;  // cell 1 from cell 0
-    double c0 = Xin[e], c1 = Xin[e + d1];
-    double xb0 = Xin[e - pl], xb1 = Xin[e - pl + d1];
-    if (k0 == 0) {
-        xb0 = ghost_f64(bc, 4, c0);
-        xb1 = ghost_f64(bc, 4, c1);
+    auto off = [&](int m) { return m < nc ? m : 0; };  // a missing cell reads the first one's values
+    double xc[NC], xb[NC], qB[NC];
+#pragma unroll
+    for (int m = 0; m < NC; ++m) {
+        xc[m] = Xin[e + off(m)];
+        xb[m] = k0 == 0 ? ghost_f64(bc, 4, xc[m]) : Xin[e - pl + off(m)];
+        qB[m] = -kz[c + off(m)] * (_dz * (xc[m] - xb[m]));
     }
-    double qB0 = -kz[c] * (_dz * (c0 - xb0)), qB1 = -kz[c + d1] * (_dz * (c1 - xb1));
     for (int k = k0; k < k1; ++k) {
+        const int par = k & 1;
         // the plane's loads first: they are in flight while the fluxes wait for the FP64 pipe
-        double f0x = Xin[e + pl], f1x = Xin[e + pl + d1], xs0 = Xin[e - n1], xs1 = Xin[e - n1 + d1], xw = Xin[e - 1];
-        const double kW0 = kx[fx], kW1 = kx[fx + 1], kS0 = ky[fy], kS1 = ky[fy + d1], kF0 = kz[c + cpl],
-                     kF1 = kz[c + cpl + d1], p0 = PC[c], p1 = PC[c + d1], m0 = F0[c], m1 = F0[c + d1];
-        double fu0 = R[c], fu1 = R[c + d1], y0 = 0.0, y1 = 0.0;
-        if (INV) {
-            y0 = iPC[c];
-            y1 = iPC[c + d1];
+        double xf[NC], xs[NC], kW[NC], kS[NC], kF[NC], pc[NC], ip[NC], mo[NC], fu[NC];
+        double xw = Xin[e - 1];
+#pragma unroll
+        for (int m = 0; m < NC; ++m) {
+            xf[m] = Xin[e + pl + off(m)];
+            xs[m] = Xin[e - n1 + off(m)];
+            kW[m] = kx[fx + (i + m <= nx ? m : 0)];
+            kS[m] = ky[fy + off(m)];
+            kF[m] = kz[c + cpl + off(m)];
+            pc[m] = PC[c + off(m)];
+            ip[m] = INV ? iPC[c + off(m)] : 0.0;
+            mo[m] = F0[c + off(m)];
+            fu[m] = R[c + off(m)];
         }
-        if (k == nz - 1) {
-            f0x = ghost_f64(bc, 5, c0);
-            f1x = ghost_f64(bc, 5, c1);
+        if (k == nz - 1)
+#pragma unroll
+            for (int m = 0; m < NC; ++m) xf[m] = ghost_f64(bc, 5, xc[m]);
+        if (j == 0)
+#pragma unroll
+            for (int m = 0; m < NC; ++m) xs[m] = ghost_f64(bc, 2, xc[m]);
+        if (i == 0) xw = ghost_f64(bc, 0, xc[0]);
+        // a cell after the row's last one stands for the wall's ghost, so the wall's flux is its west flux
+        double a[NC + 1], xe = 0.0;
+        a[0] = xw;
+#pragma unroll
+        for (int m = 0; m < NC; ++m) {
+            a[m + 1] = xc[m];
+            if (m > 0 && i + m == nx) a[m + 1] = xe = ghost_f64(bc, 1, xc[m - 1]);
         }
-        if (j == 0) {
-            xs0 = ghost_f64(bc, 2, c0);
-            xs1 = ghost_f64(bc, 2, c1);
+        double qx[NC + 1], qS[NC], qN[NC], qF[NC];
+#pragma unroll
+        for (int m = 0; m < NC; ++m) {
+            qx[m] = -kW[m] * (_dx * (a[m + 1] - a[m]));
+            qS[m] = -kS[m] * (_dy * (xc[m] - xs[m]));
+            south[par][m][tid] = qS[m];
         }
-        if (i == 0) xw = ghost_f64(bc, 0, c0);
-        double a1 = c1, xe = 0.0;
-        if (!in1) a1 = xe = ghost_f64(bc, 1, c0);  // cell 0 is the row's last: its east wall as cell 1's west face
-        const double qW0 = -kW0 * (_dx * (c0 - xw)), qW1 = -kW1 * (_dx * (a1 - c0));
-        const double qS0 = -kS0 * (_dy * (c0 - xs0)), qS1 = -kS1 * (_dy * (c1 - xs1));
-        west[k & 1][tid] = qW0;
-        south[k & 1][tid] = make_double2(qS0, qS1);
-        const double z0 = -kF0 * (_dz * (f0x - c0)), z1 = -kF1 * (_dz * (f1x - c1));
+        west[par][tid] = qx[0];
+#pragma unroll
+        for (int m = 0; m < NC; ++m) qF[m] = -kF[m] * (_dz * (xf[m] - xc[m]));
         __syncthreads();
-        double qE1 = 0.0, qN0, qN1, xn0 = 0.0, xn1 = 0.0;
+        qx[NC] = 0.0;
         if (east_here) {
-            xe = i + 2 == nx ? ghost_f64(bc, 1, c1) : Xin[e + 2];
-            qE1 = -kx[fx + 2] * (_dx * (xe - c1));
+            xe = wall ? ghost_f64(bc, 1, xc[NC - 1]) : Xin[e + NC];
+            qx[NC] = -kx[fx + NC] * (_dx * (xe - xc[NC - 1]));
         } else if (tid + 1 < T) {
-            qE1 = west[k & 1][tid + 1];
+            qx[NC] = west[par][tid + 1];
         }
+        double xn[NC];
         if (north_here) {
-            xn0 = j >= ny - 1 ? ghost_f64(bc, 3, c0) : Xin[e + n1];
-            xn1 = j >= ny - 1 ? ghost_f64(bc, 3, c1) : Xin[e + n1 + d1];
-            qN0 = -ky[fy + nx] * (_dy * (xn0 - c0));
-            qN1 = -ky[fy + nx + d1] * (_dy * (xn1 - c1));
-        } else {
-            const double2 n = south[k & 1][tid + np];
-            qN0 = n.x;
-            qN1 = n.y;
-        }
-        if (CX) {
-            fu0 = fu0 + s.cX * c0;
-            fu1 = fu1 + s.cX * c1;
-        }
-        fu0 = fu0 + _dx * (qW1 - qW0) + _dy * (qN0 - qS0) + _dz * (z0 - qB0);
-        fu1 = fu1 + _dx * (qE1 - qW1) + _dy * (qN1 - qS1) + _dz * (z1 - qB1);
-        const double f0 = INV ? div_known(fu0, p0, y0) : div_any(fu0, p0);
-        const double f1 = INV ? div_known(fu1, p1, y1) : div_any(fu1, p1);
-        const double g0 = h1 * m0 + h2 * f0, g1 = h1 * m1 + h2 * f1;
-        const double r0 = dtau * g0, r1 = dtau * g1;
-        const double o0 = c0 - r0, o1 = c1 - r1;
-        if (row) {
-            F0[c] = g0;
-            Xout[e] = o0;
-            if (in1) {
-                F0[c + 1] = g1;
-                Xout[e + 1] = o1;
+#pragma unroll
+            for (int m = 0; m < NC; ++m) {
+                xn[m] = j >= ny - 1 ? ghost_f64(bc, 3, xc[m]) : Xin[e + n1 + off(m)];
+                qN[m] = -ky[fy + nx + off(m)] * (_dy * (xn[m] - xc[m]));
             }
+        } else {
+#pragma unroll
+            for (int m = 0; m < NC; ++m) qN[m] = south[par][m][tid + np];
+        }
+#pragma unroll
+        for (int m = 0; m < NC; ++m) {
+            if (CX) fu[m] = fu[m] + s.cX * xc[m];
+            fu[m] = fu[m] + _dx * (qx[m + 1] - qx[m]) + _dy * (qN[m] - qS[m]) + _dz * (qF[m] - qB[m]);
+            const double f = INV ? div_known(fu[m], pc[m], ip[m]) : div_any(fu[m], pc[m]);
+            const double f0 = h1 * mo[m] + h2 * f;
+            const double d = dtau * f0;
+            const double o = xc[m] - d;
+            if (!row || m >= nc) continue;
+            F0[c + m] = f0;
+            Xout[e + m] = o;
             if (MODE == MODE_CHECK) {  // per-cell terms of the check sums (canonical tree order)
                 const long long n = (long long)cpl * nz;
-                partials[c] = fabs(f0 * p0);
-                partials[c + n] = -r0 * (f0 - F[c]);
-                partials[c + 2 * n] = r0 * r0;
-                if (in1) {
-                    partials[c + 1] = fabs(f1 * p1);
-                    partials[c + 1 + n] = -r1 * (f1 - F[c + 1]);
-                    partials[c + 1 + 2 * n] = r1 * r1;
-                }
+                partials[c + m] = fabs(f * pc[m]);
+                partials[c + m + n] = -d * (f - F[c + m]);
+                partials[c + m + 2 * n] = d * d;
             }
-            if (MODE >= MODE_STOREF) {
-                F[c] = f0;
-                if (in1) F[c + 1] = f1;
-            }
+            if (MODE >= MODE_STOREF) F[c + m] = f;
             // face ghosts of the output = BC of the input (reference state)
-            if (i == 0) Xout[e - 1] = xw;
-            if (!in1) Xout[e + 1] = xe;
-            if (i + 2 == nx) Xout[e + 2] = xe;
-            if (j == 0) {
-                Xout[e - n1] = xs0;
-                if (in1) Xout[e - n1 + 1] = xs1;
-            }
-            if (j == ny - 1) {
-                Xout[e + n1] = xn0;
-                if (in1) Xout[e + n1 + 1] = xn1;
-            }
-            if (k == 0) {
-                Xout[e - pl] = xb0;
-                if (in1) Xout[e - pl + 1] = xb1;
-            }
-            if (k == nz - 1) {
-                Xout[e + pl] = f0x;
-                if (in1) Xout[e + pl + 1] = f1x;
-            }
+            if (i + m == 0) Xout[e - 1] = xw;
+            if (i + m == nx - 1) Xout[e + m + 1] = xe;
+            if (j == 0) Xout[e + m - n1] = xs[m];
+            if (j == ny - 1) Xout[e + m + n1] = xn[m];
+            if (k == 0) Xout[e + m - pl] = xb[m];
+            if (k == nz - 1) Xout[e + m + pl] = xf[m];
         }
-        c0 = f0x;
-        c1 = f1x;
-        qB0 = z0;
-        qB1 = z1;
+#pragma unroll
+        for (int m = 0; m < NC; ++m) {
+            xc[m] = xf[m];
+            qB[m] = qF[m];
+        }
         e += pl;
         c += cpl;
         fx += (nx + 1) * ny;
@@ -177,28 +171,24 @@ __global__ void k_reciprocal(double* __restrict__ iPC, const double* __restrict_
 }
 
 struct F64Launch {
-    int threads, zchunk;
+    int cells, threads, zchunk;  // cells per thread, threads per block, planes per block
     dim3 grid;
 };
-// Chunks of planes so that the SMs carry about the same number of planes (a
-// block's time is its planes' plus a tenth for the first one's extra flux).  256
-// threads keep two warps per scheduler busy with one block per SM; small grids
-// spread over more schedulers with 128.
-inline F64Launch f64_launch(int sms, int nx, int ny, int nz) {
-    F64Launch L;
-    const long long pairs = (long long)((nx + 1) / 2) * ny;
-    L.threads = pairs * nz >= 256LL * sms ? 256 : 128;
-    const long long gx = (pairs + L.threads - 1) / L.threads;
-    long long best = -1;
-    for (int c = 1; c <= std::min(nz, 64); ++c) {
-        const long long blocks = gx * ((nz + c - 1) / c);
-        // blocks in a row on an SM, in halves; where there are many, the last wave is half full
-        const long long deep = blocks >= 4LL * sms ? 2 * blocks / sms + 1 : 2 * ((blocks + sms - 1) / sms);
-        const long long cost = deep * (10LL * c + 1);
-        if (best < 0 || cost < best) best = cost, L.zchunk = c;
-    }
-    L.grid = dim3((unsigned)gx, 1, (nz + L.zchunk - 1) / L.zchunk);
-    return L;
+inline F64Launch f64_shape(int cells, int threads, int zchunk, int nx, int ny, int nz) {
+    const long long runs = (long long)((nx + cells - 1) / cells) * ny;
+    return F64Launch{cells, threads, zchunk,
+                     dim3((unsigned)((runs + threads - 1) / threads), 1, (unsigned)((nz + zchunk - 1) / zchunk))};
+}
+// Small grids: a cell per thread and a plane per block, as many warps as there
+// are (31 x 29 x 33: 4.9 us, 6.0 with two planes, 5.0 with two cells).  From 2^16
+// cells on two cells per thread, and chunks that leave each SM several blocks,
+// since one block's waits are hidden by another's arithmetic: two planes up to
+// 2^19 cells (63^3: 20.6 us, three 29), three up to 2^22 (95^3: 58.5, two 60.0;
+// 127 x 119 x 131: 131, two 138), eight above (255^3: 1009, three 1037).
+inline F64Launch f64_launch(int nx, int ny, int nz) {
+    const long long n = (long long)nx * ny * nz;
+    if (n < (1LL << 16)) return f64_shape(1, 128, 1, nx, ny, nz);
+    return f64_shape(2, 256, n < (1LL << 19) ? 2 : (n < (1LL << 22) ? 3 : 8), nx, ny, nz);
 }
 
 template <int MODE>
@@ -206,12 +196,12 @@ struct F64Kernel {
     typedef void (*Fn)(const double*, double*, const double*, const double*, const double*, const double*, const double*,
                        const double*, double*, double*, DyrelScalT<double>, BC6<double>, int, int, int, int, double*);
     template <bool CX, bool INV>
-    static Fn by_size(int threads) {
-        return threads == 256 ? (Fn)k_dyrel_f64<MODE, CX, INV, 256> : (Fn)k_dyrel_f64<MODE, CX, INV, 128>;
+    static Fn by_shape(const F64Launch& L) {
+        return L.cells == 1 ? (Fn)k_dyrel_f64<MODE, CX, INV, 128, 1> : (Fn)k_dyrel_f64<MODE, CX, INV, 256, 2>;
     }
-    static Fn get(bool cx, bool inv, int threads) {
-        return cx ? (inv ? by_size<true, true>(threads) : by_size<true, false>(threads))
-                  : (inv ? by_size<false, true>(threads) : by_size<false, false>(threads));
+    static Fn get(bool cx, bool inv, const F64Launch& L) {
+        return cx ? (inv ? by_shape<true, true>(L) : by_shape<true, false>(L))
+                  : (inv ? by_shape<false, true>(L) : by_shape<false, false>(L));
     }
 };
 

@@ -15,7 +15,7 @@ int ht3d_dyrel_solve_fp64(ht3d_ctx* ctx, double* X, const double* R, const doubl
     double* X2 = (double*)ht3d_scratch(ctx, SLOT_X2, sizeof(double) * nex);
     IterLaunch L = iter_launch(ctx, nx, ny, nz);
     const bool fixed_variant = ctx->dyrel_variant != 0;  // the caller's thread layout
-    const F64Launch L64 = f64_launch(ctx->num_sms, nx, ny, nz);
+    const F64Launch L64 = f64_launch(nx, ny, nz);
     double* iPC = fixed_variant ? nullptr : (double*)ht3d_scratch(ctx, SLOT_G, sizeof(double) * n);
     const long long nsetup = (long long)((nx + 31) / 32) * ((ny + 7) / 8) * nz;
     // per-cell check terms (3n) followed by tree-pass work space
@@ -62,11 +62,11 @@ int ht3d_dyrel_solve_fp64(ht3d_ctx* ctx, double* X, const double* R, const doubl
         sc.dtau = S.dtau;
         if (iPC) {
             const bool cx = cX != 0.0;
-            const auto kern = chk ? F64Kernel<MODE_CHECK>::get(cx, true, L64.threads)
-                                  : (storef ? F64Kernel<MODE_STOREF>::get(cx, true, L64.threads)
-                                            : F64Kernel<MODE_PLAIN>::get(cx, true, L64.threads));
-            HT3D_LAUNCH(ctx, kern, L64.grid, L64.threads, 0, cur, nxt, R, kx, ky, kz, PC, iPC, F0, F,
-                        DyrelScalT<double>(sc), bc, nx, ny, nz, L64.zchunk, parts);
+            const auto kern = chk ? F64Kernel<MODE_CHECK>::get(cx, true, L64)
+                                  : (storef ? F64Kernel<MODE_STOREF>::get(cx, true, L64)
+                                            : F64Kernel<MODE_PLAIN>::get(cx, true, L64));
+            launch_after(ctx, kern, L64.grid, L64.threads, 0, cur, nxt, R, kx, ky, kz, PC, iPC, F0, F,
+                         DyrelScalT<double>(sc), bc, nx, ny, nz, L64.zchunk, parts);
         } else if (chk)
             launch_iter<double, MODE_CHECK>(ctx, L, cur, nxt, R, kx, ky, kz, PC, F0, F, sc, bc, nx, ny, nz, parts);
         else if (storef)
@@ -142,14 +142,14 @@ extern "C" int ht3d_dyrel_iterate(ht3d_ctx* ctx, double* X_ex, const double* R, 
             iPC = (double*)ht3d_scratch(ctx, SLOT_G, sizeof(double) * n);
             HT3D_LAUNCH(ctx, k_reciprocal, (unsigned)std::min<long long>((n + 255) / 256, ctx->num_sms * 16LL), 256, 0, iPC, PC, n);
         }
-        const F64Launch L = f64_launch(ctx->num_sms, nx, ny, nz);
+        const F64Launch L = f64_launch(nx, ny, nz);
         const DyrelScalT<double> sc(DyrelScal{h1, h2, dtau, cX, 1.0 / dx, 1.0 / dy, 1.0 / dz});
-        const auto kern = F64Kernel<MODE_PLAIN>::get(cX != 0.0, iPC != nullptr, L.threads);
+        const auto kern = F64Kernel<MODE_PLAIN>::get(cX != 0.0, iPC != nullptr, L);
         double* cur = X_ex;
         double* nxt = X2;
         for (int it = 0; it < n_iter; ++it) {
-            HT3D_LAUNCH(ctx, kern, L.grid, L.threads, 0, cur, nxt, R, kx, ky, kz, PC, iPC, F0, (double*)nullptr, sc,
-                        bc, nx, ny, nz, L.zchunk, (double*)nullptr);
+            launch_after(ctx, kern, L.grid, L.threads, 0, cur, nxt, R, kx, ky, kz, PC, iPC, F0, (double*)nullptr, sc,
+                         bc, nx, ny, nz, L.zchunk, (double*)nullptr);
             std::swap(cur, nxt);
         }
         if (cur != X_ex) {

@@ -136,6 +136,31 @@ static inline bool all_nonnull(P... p) {
         (ctx)->launches++;                                                     \
     } while (0)
 
+// A launch that may be set up while the kernel before it in the stream still
+// runs (programmatic dependent launch).  The kernel calls after_previous()
+// before it touches memory, which waits until the launches before it are
+// complete and their writes visible: the same order as plain launches, without
+// the gap between two kernels.
+__device__ __forceinline__ void after_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... P, typename... A>
+static inline void launch_after(ht3d_ctx* ctx, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    HT3D_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
+    ctx->launches++;
+}
+
 // Phase codes (-1 immersed, 0 crust, 1 air, 2 fault, 3 pluton) are small
 // integers stored as doubles.  Equality with a nonzero code is tested on the
 // bit pattern: the same truth value as the FP64 comparison for every input,

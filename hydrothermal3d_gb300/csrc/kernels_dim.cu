@@ -495,9 +495,9 @@ int ht3d_material_law(ht3d_ctx* ctx, int which, const double* a, const double* b
 // reading the snapshot X_in and writing the updated inner cells of X_out.
 // The boundary rules are evaluated on the fly for every stencil point
 // (bc_value below, the rules of k_dim_bcs in order); the ghost shell of X_out
-// is written by k_dim_shell.  Phase codes are read as int8.
+// is written by the launch's last blocks.  Phase codes are read as int8.
 // ===========================================================================
-#include "dyrel_common.cuh"
+#include "dyrel_f64.cuh"
 
 void ht3d_weno5_advect_impl(ht3d_ctx* ctx, double* Tc_ex, const double* Vx, const double* Vy, const double* Vz,
                             double dt, double _dx, double _dy, double _dz, const int* bc_type6, const double* bc_val6,
@@ -537,22 +537,6 @@ __device__ __forceinline__ double bc_value(const double* __restrict__ S, const s
     return v;
 }
 
-// ghost shell of X_out = boundary values of X_in (blockIdx.z: face pair 0 x, 1 y, 2 z)
-template <int PRESSURE>
-__global__ void k_dim_shell(double* __restrict__ Xout, const double* __restrict__ S, const signed char* __restrict__ ph,
-                            const double* __restrict__ wN, const double* __restrict__ ky, DimBC b, int nx, int ny,
-                            int nz) {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    const int c = blockIdx.y * blockDim.y + threadIdx.y;
-    const int n1 = nx + 2, n2 = ny + 2, n3 = nz + 2;
-    const int face = blockIdx.z >> 1, side = blockIdx.z & 1;
-    int i, j, k;
-    if (face == 0) { if (a >= n2 || c >= n3) return; i = side ? n1 - 1 : 0; j = a; k = c; }
-    else if (face == 1) { if (a >= n1 || c >= n3) return; i = a; j = side ? n2 - 1 : 0; k = c; }
-    else { if (a >= n1 || c >= n2) return; i = a; j = c; k = side ? n3 - 1 : 0; }
-    Xout[EXI(i, j, k)] = bc_value<PRESSURE>(S, ph, wN, ky, b, i, j, k, nx, ny, nz);
-}
-
 struct DimIterArgs {
     const double* Xin;
     double* Xout;
@@ -562,90 +546,198 @@ struct DimIterArgs {
     const double* ky;
     const double* kz;
     const double* PC;
+    const double* iPC;     // 1 / PC
     double* F0;
     double* F;
     double* terms;
     // thermal
     const double* T0;
-    const double* rC;
+    const double* rCt;     // transient rhoC / dt
     // Darcy
-    const double* Tex;     // temperature (ex) for ϕρf
     const double* prf0;    // ϕρf_old
     const double* rfy;     // av_xza(ρfv) on y faces
+    const double* tt;      // the density's temperature terms (k_rhof_terms)
 };
 
 struct DimScal {
     double h1, h2, dtau, _dx, _dy, _dz, _dt, transient, Qt, g;
     double phi_i, s_rho, s_T, s_sigma;
+    // products and reciprocals that every cell shares
+    double tQt, tdt, phi_f, y_rho;  // transient Qt, transient / dt, 3 phi_i, 1 / s_rho
 };
 
-template <int PRESSURE, int MODE>
-__global__ void __launch_bounds__(CX_* CY_* CZ_) k_dim_iter(DimIterArgs A, DimScal s, DimBC b, int nx, int ny, int nz) {
-    const int i = blockIdx.x * CX_ + threadIdx.x;
-    const int j = blockIdx.y * CY_ + threadIdx.y;
-    const int k = blockIdx.z * CZ_ + threadIdx.z;
-    if (i >= nx || j >= ny || k >= nz) return;
-    const int I = i + 1, J = j + 1, K = k + 1;
-    const int c = CI(i, j, k);
+// Terms of law_rhof_C that depend on the temperature alone, which does not
+// change during a Darcy solve, in planes of n cells: T, T^2, T^3 (in C) and the
+// polynomial's own T, T^2, T^3 and T^4 terms.
+constexpr int kRhofTerms = 7;
+__global__ void k_rhof_terms(double* __restrict__ tt, const double* __restrict__ Tex, double s_T, int nx, int ny, int nz) {
+    const long long n = (long long)nx * ny * nz;
+    for_cells_z(nx, ny, nz, [&](int i, int j, int k) {
+        const long long c = CI(i, j, k);
+        const double T_C = Tex[EXI(i + 1, j + 1, k + 1)] * s_T - 273.15;
+        const double T2 = T_C * T_C, T3 = T_C * T_C * T_C, T4 = T2 * T2;
+        const double v[kRhofTerms] = {T_C, T2, T3, -0.3922 * T_C, -0.003774 * T2, 2.955e-6 * T3, 5.698e-11 * T4};
+#pragma unroll
+        for (int q = 0; q < kRhofTerms; ++q) tt[c + q * n] = v[q];
+    });
+}
+// law_rhof_C (laws.cuh), statement for statement, with those terms at hand
+__device__ __forceinline__ double rhof_from_terms(const double (&t)[kRhofTerms], double p) {
+    const double p2 = p * p, p3 = p * p * p, p4 = p2 * p2;
+    return 1006 + (7.424e-7 * p) + t[3] + (-4.441e-15 * p2) + (4.547e-9 * p * t[0]) + t[4] + (1.451e-23 * p3) +
+           (-1.793e-17 * p2 * t[0]) + (7.485e-12 * p * t[1]) + t[5] + (-1.463e-32 * p4) + (1.361e-26 * p3 * t[0]) +
+           (4.018e-21 * (p2) * (t[1])) + (-7.372e-15 * p * t[2]) + t[6];
+}
+// thermal: transient rhoC / dt of every cell
+__global__ void k_scale_rc(double* __restrict__ out, const double* __restrict__ rC, double transient, double _dt, long long n) {
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
+        out[t] = transient * rC[t] * _dt;
+}
+
+// One pseudo-iteration on the layout of k_dyrel_f64 (dyrel_f64.cuh: pairs of
+// cells, fluxes evaluated once and handed on in shared memory), FP64-bound like
+// it: about 70 operations per cell for Darcy instead of 104 and 30 instead of 47
+// for heat, which also evaluated every flux twice and divided by the operator;
+// the density's temperature terms come from memory.  The last blocks write the
+// ghost shell of X_out (boundary values of X_in), which took a launch of its own.
+// TRANS: the Darcy residual has its storage term (0 times a finite term adds
+// nothing).  us per iteration with the shell, before and now, heat and Darcy:
+// 24 x 24 x 12 12.3 -> 5.5 and 16.4 -> 6.9, 63^3 32.8 -> 22.7 and 59.4 -> 41.9,
+// 127^3 192 -> 152 and 403 -> 307.
+template <int PRESSURE, int MODE, bool TRANS, int T, int NC>
+__global__ void __launch_bounds__(T) k_dim_iter(DimIterArgs A, DimScal s, DimBC b, int nx, int ny, int nz, int zchunk,
+                                                int work_blocks, int cell_blocks) {
+    after_previous();
+    const int n1 = nx + 2, n2 = ny + 2, n3 = nz + 2;
+    const int tid = threadIdx.x;
+    if ((int)blockIdx.x >= work_blocks) {
+        long long t = (long long)((int)blockIdx.x - work_blocks) * T + tid;
+        const long long fx = (long long)n2 * n3, fy = (long long)n1 * n3, fz = (long long)n1 * n2;
+        int i, j, k;
+        if (t < 2 * fx) {
+            i = t < fx ? 0 : n1 - 1;
+            t = t < fx ? t : t - fx;
+            j = (int)(t % n2);
+            k = (int)(t / n2);
+        } else if (t < 2 * (fx + fy)) {
+            t -= 2 * fx;
+            j = t < fy ? 0 : n2 - 1;
+            t = t < fy ? t : t - fy;
+            i = (int)(t % n1);
+            k = (int)(t / n1);
+        } else if (t < 2 * (fx + fy + fz)) {
+            t -= 2 * (fx + fy);
+            k = t < fz ? 0 : n3 - 1;
+            t = t < fz ? t : t - fz;
+            i = (int)(t % n1);
+            j = (int)(t / n1);
+        } else {
+            return;
+        }
+        A.Xout[EXI(i, j, k)] = bc_value<PRESSURE>(A.Xin, A.ph, A.wN, A.ky, b, i, j, k, nx, ny, nz);
+        return;
+    }
+    __shared__ double west[2][T], south[2][NC][T];
+    const int blk = (int)blockIdx.x, bz = blk / cell_blocks, np = (nx + NC - 1) / NC;
+    const int t = (blk - bz * cell_blocks) * T + tid;
+    const int j = t / np, i = NC * (t - j * np);
+    const bool row = j < ny;
+    const int k0 = bz * zchunk, k1 = min(nz, k0 + zchunk);
+    const int J = min(j, ny - 1) + 1, I = i + 1;  // threads past the plane read its last row and store nothing
+    const int nc = min(NC, nx - i);                                                // cells of this thread
+    const bool east_here = i + NC == nx || (tid == T - 1 && i + NC < nx);          // no thread's west face
+    const bool north_here = j >= ny - 1 || tid + np >= T;
+    const int pl = n1 * n2, cpl = nx * ny;
+    auto off = [&](int m) { return m < nc ? m : 0; };  // a missing cell reads the first one's values
     auto X = [&](int ii, int jj, int kk) {
         return bc_value<PRESSURE>(A.Xin, A.ph, A.wN, A.ky, b, ii, jj, kk, nx, ny, nz);
     };
-    const double xc = X(I, J, K);
-    const double xw = X(I - 1, J, K), xe = X(I + 1, J, K);
-    const double xs = X(I, J - 1, K), xn = X(I, J + 1, K);
-    const double xb = X(I, J, K - 1), xf = X(I, J, K + 1);
-    const int fx = ix3(i, j, k, nx + 1, ny), fy = ix3(i, j, k, nx, ny + 1);
-    const double qW = -A.kx[fx] * (s._dx * (xc - xw));
-    const double qE = -A.kx[fx + 1] * (s._dx * (xe - xc));
-    const double qB = -A.kz[c] * (s._dz * (xc - xb));
-    const double qF = -A.kz[c + nx * ny] * (s._dz * (xf - xc));
-    double qS, qN;
-    if (PRESSURE) {
-        qS = -A.ky[fy] * (s._dy * (xc - xs) - s.g * A.rfy[fy]);
-        qN = -A.ky[fy + nx] * (s._dy * (xn - xc) - s.g * A.rfy[fy + nx]);
-    } else {
-        qS = -A.ky[fy] * (s._dy * (xc - xs));
-        qN = -A.ky[fy + nx] * (s._dy * (xn - xc));
+    // y flux through face f (of the faces' array) from the values south and north of it
+    auto flux_y = [&](int f, double lo, double hi) {
+        return PRESSURE ? -A.ky[f] * (s._dy * (hi - lo) - s.g * A.rfy[f]) : -A.ky[f] * (s._dy * (hi - lo));
+    };
+    int e = EXI(I, J, k0 + 1), c = CI(i, J - 1, k0);
+    int fx = ix3(i, J - 1, k0, nx + 1, ny), fy = ix3(i, J - 1, k0, nx, ny + 1);
+    double xc[NC], qB[NC];
+#pragma unroll
+    for (int m = 0; m < NC; ++m) {
+        xc[m] = X(I + off(m), J, k0 + 1);
+        qB[m] = -A.kz[c + off(m)] * (s._dz * (xc[m] - X(I + off(m), J, k0)));
     }
-    const int e = EXI(I, J, K);
-    const int p = A.ph[e];
-    double f = 0.;
-    if (p != 1 && p != -1) {
-        if (PRESSURE) {
-            // ϕρf from the pre-boundary-kernel pressure (the reference runs ϕρf first)
-            const double Tc = A.Tex[e] * s.s_T - 273.15;
-            const double Pc = A.Xin[e] * s.s_sigma;
-            const double prf = law_phi((double)p, s.phi_i) * law_rhof_C(Tc, Pc) / s.s_rho;
-            f = s.transient * s._dt * (prf - A.prf0[c]);
+    const long long n = (long long)cpl * nz;
+    for (int k = k0; k < k1; ++k) {
+        const int K = k + 1, par = k & 1;
+        double xf[NC], a[NC + 1], qx[NC + 1], qS[NC], qN[NC], qF[NC];
+        a[0] = X(I - 1, J, K);
+#pragma unroll
+        for (int m = 0; m < NC; ++m) {
+            xf[m] = X(I + off(m), J, K + 1);
+            // a cell after the row's last one stands for the ghost, so the wall's flux is its west flux
+            a[m + 1] = m > 0 && i + m == nx ? X(I + m, J, K) : xc[m];
+            qx[m] = -A.kx[fx + (i + m <= nx ? m : 0)] * (s._dx * (a[m + 1] - a[m]));
+            qS[m] = flux_y(fy + off(m), X(I + off(m), J - 1, K), xc[m]);
+            qF[m] = -A.kz[c + cpl + off(m)] * (s._dz * (xf[m] - xc[m]));
+            south[par][m][tid] = qS[m];
+        }
+        west[par][tid] = qx[0];
+        __syncthreads();
+        qx[NC] = 0.0;
+        if (east_here) qx[NC] = -A.kx[fx + NC] * (s._dx * (X(I + NC, J, K) - xc[NC - 1]));
+        else if (tid + 1 < T) qx[NC] = west[par][tid + 1];
+        if (north_here) {
+#pragma unroll
+            for (int m = 0; m < NC; ++m) qN[m] = flux_y(fy + nx + off(m), xc[m], X(I + off(m), J + 1, K));
         } else {
-            double Q = 0.;
-            if (p == 3) Q = s.Qt;
-            f = s.transient * A.rC[c] * s._dt * (xc - A.T0[c]);
-            f += (qE - qW) * s._dx;
-            f += (qN - qS) * s._dy;
-            f += (qF - qB) * s._dz;
-            f -= s.transient * Q;
-            f /= A.PC[c];
+#pragma unroll
+            for (int m = 0; m < NC; ++m) qN[m] = south[par][m][tid + np];
         }
-        if (PRESSURE) {
-            f += (qE - qW) * s._dx;
-            f += (qN - qS) * s._dy;
-            f += (qF - qB) * s._dz;
-            f /= A.PC[c];
+#pragma unroll
+        for (int m = 0; m < NC; ++m) {
+            const int cc = c + off(m), p = A.ph[e + off(m)];
+            double f = 0.;
+            if (PRESSURE) {
+                if (TRANS) {
+                    // ϕρf from the pre-boundary-kernel pressure (the reference runs ϕρf first)
+                    double tt[kRhofTerms];
+#pragma unroll
+                    for (int r = 0; r < kRhofTerms; ++r) tt[r] = A.tt[cc + r * n];
+                    const double rho = rhof_from_terms(tt, A.Xin[e + off(m)] * s.s_sigma);
+                    const double prf = div_known((p == 2 ? s.phi_f : s.phi_i) * rho, s.s_rho, s.y_rho);
+                    f = s.tdt * (prf - A.prf0[cc]);
+                }
+            } else {
+                f = A.rCt[cc] * (xc[m] - A.T0[cc]);
+            }
+            f += (qx[m + 1] - qx[m]) * s._dx;
+            f += (qN[m] - qS[m]) * s._dy;
+            f += (qF[m] - qB[m]) * s._dz;
+            if (!PRESSURE && p == 3) f -= s.tQt;
+            const double pc = A.PC[cc];
+            f = div_known(f, pc, A.iPC[cc]);
+            if (p == 1 || p == -1) f = 0.;
+            const double f0 = s.h1 * A.F0[cc] + s.h2 * f;
+            const double d = s.dtau * f0;
+            const double o = xc[m] - d;
+            if (!row || m >= nc) continue;
+            A.F0[cc] = f0;
+            A.Xout[e + m] = o;
+            if (MODE == MODE_CHECK) {
+                A.terms[cc] = fabs(f * pc);
+                A.terms[cc + n] = -d * (f - A.F[cc]);
+                A.terms[cc + 2 * n] = d * d;
+            }
+            if (MODE >= MODE_STOREF) A.F[cc] = f;
         }
+#pragma unroll
+        for (int m = 0; m < NC; ++m) {
+            xc[m] = xf[m];
+            qB[m] = qF[m];
+        }
+        e += pl;
+        c += cpl;
+        fx += (nx + 1) * ny;
+        fy += nx * (ny + 1);
     }
-    const double f0 = s.h1 * A.F0[c] + s.h2 * f;
-    A.F0[c] = f0;
-    A.Xout[e] = xc - s.dtau * f0;
-    if (MODE == MODE_CHECK) {
-        const double fit = A.F[c];
-        const double d = s.dtau * f0;
-        const int n = nx * ny * nz;
-        A.terms[c] = fabs(f * A.PC[c]);
-        A.terms[c + n] = -d * (f - fit);
-        A.terms[c + 2 * n] = d * d;
-    }
-    if (MODE >= MODE_STOREF) A.F[c] = f;
 }
 
 __global__ void k_pluton(double* T, const double* __restrict__ phc, double Tp, long long n) {
@@ -680,8 +772,33 @@ __global__ void k_gersh(double* G, double* D, const double* __restrict__ rC, con
     G[CI(i, j, k)] = g / diag;
 }
 
+// blocks of `threads` that cover the ghost shell (edges twice)
+inline long long shell_blocks(int threads, int nx, int ny, int nz) {
+    const long long n1 = nx + 2, n2 = ny + 2, n3 = nz + 2;
+    return (2 * (n2 * n3 + n1 * n3 + n1 * n2) + threads - 1) / threads;
+}
+// A cell per thread below 2^20 cells (63^3, Darcy: 41.9 us, 45.7 with two), and
+// the chunk for which the SMs' last blocks end together: a block's time is about
+// its planes and a third of one (48 x 48 x 24, Darcy: one plane 16.8 us, two
+// 14.8; 56 x 56 x 28: 17.4 and 30.2).  Two cells above (127^3, heat: 152 us, 161
+// with one), in chunks of two planes or, with blocks to spare, eight.
+inline F64Launch dim_launch(int sms, int nx, int ny, int nz) {
+    const long long n = (long long)nx * ny * nz;
+    if (n >= (1LL << 20)) return f64_shape(2, 256, n < (1LL << 22) ? 2 : 8, nx, ny, nz);
+    F64Launch best = f64_shape(1, 128, 1, nx, ny, nz);
+    long long least = -1;
+    for (int c = 1; c <= 4; ++c) {
+        const F64Launch L = f64_shape(1, 128, c, nx, ny, nz);
+        const long long blocks = (long long)L.grid.x * L.grid.z + shell_blocks(128, nx, ny, nz);
+        const long long cost = (blocks + sms - 1) / sms * (3 * c + 1);
+        if (least < 0 || cost < least) least = cost, best = L;
+    }
+    return best;
+}
+
 struct DimWork {
     double *X2, *kv, *dumc, *kx, *ky, *kz, *rC, *PC, *G, *F, *F0, *T0, *P0, *rfy, *terms, *prf0;
+    double *iPC, *tt;   // 1 / PC; the Darcy iteration's temperature terms, or the heat's rhoC factor
     const double* Tex;  // temperature (ex) read by the Darcy iteration
     signed char* ph;
 };
@@ -699,12 +816,35 @@ int dim_dyrel(ht3d_ctx* ctx, double* X, DimWork& W, const double* wN, DimScal s,
     HT3D_CUDA(cudaMemsetAsync(W.F0, 0, sizeof(double) * n, ctx->stream));
     // both buffers start identical so cells no rule writes stay equal
     HT3D_CUDA(cudaMemcpyAsync(W.X2, X, sizeof(double) * nex, cudaMemcpyDeviceToDevice, ctx->stream));
-    const dim3 blk(CX_, CY_, CZ_), grd((nx + CX_ - 1) / CX_, (ny + CY_ - 1) / CY_, (nz + CZ_ - 1) / CZ_);
-    const int nm = std::max(nx, std::max(ny, nz)) + 2;
-    const dim3 sb(32, 8, 1), sg((nm + 31) / 32, (nm + 7) / 8, 6);
+    s.tQt = s.transient * s.Qt;
+    s.tdt = s.transient * s._dt;
+    s.phi_f = 3 * s.phi_i;
+    s.y_rho = 1.0 / s.s_rho;
+    const unsigned g1 = (unsigned)std::max<long long>(1, std::min<long long>((n + 255) / 256, ctx->num_sms * 16LL));
+    HT3D_LAUNCH(ctx, k_reciprocal, g1, 256, 0, W.iPC, W.PC, n);
+    const bool trans = s.tdt != 0.0;
+    if (!PRESSURE) HT3D_LAUNCH(ctx, k_scale_rc, g1, 256, 0, W.tt, W.rC, s.transient, s._dt, n);
+    else if (trans) HT3D_LAUNCH(ctx, k_rhof_terms, grid3z(nx, ny, nz), kBlock3, 0, W.tt, W.Tex, s.s_T, nx, ny, nz);
+    const F64Launch L = dim_launch(ctx->num_sms, nx, ny, nz);
+    const int cb = (int)L.grid.x, wb = (int)(cb * L.grid.z);
+    const unsigned grd = (unsigned)(wb + shell_blocks(L.threads, nx, ny, nz));
+    typedef void (*Kern)(DimIterArgs, DimScal, DimBC, int, int, int, int, int, int);
+    auto kern_of = [&](auto tr, int mode) -> Kern {
+        constexpr bool TR = decltype(tr)::value;
+        if (L.cells == 1)
+            return mode == MODE_CHECK ? (Kern)k_dim_iter<PRESSURE, MODE_CHECK, TR, 128, 1>
+                                      : (mode == MODE_STOREF ? (Kern)k_dim_iter<PRESSURE, MODE_STOREF, TR, 128, 1>
+                                                             : (Kern)k_dim_iter<PRESSURE, MODE_PLAIN, TR, 128, 1>);
+        return mode == MODE_CHECK ? (Kern)k_dim_iter<PRESSURE, MODE_CHECK, TR, 256, 2>
+                                  : (mode == MODE_STOREF ? (Kern)k_dim_iter<PRESSURE, MODE_STOREF, TR, 256, 2>
+                                                         : (Kern)k_dim_iter<PRESSURE, MODE_PLAIN, TR, 256, 2>);
+    };
+    auto pick = [&](int mode) {
+        return PRESSURE && trans ? kern_of(std::bool_constant<PRESSURE != 0>(), mode) : kern_of(std::false_type(), mode);
+    };
     DimIterArgs A;
-    A.ph = W.ph; A.wN = wN; A.kx = W.kx; A.ky = W.ky; A.kz = W.kz; A.PC = W.PC; A.F0 = W.F0; A.F = W.F;
-    A.terms = W.terms; A.T0 = W.T0; A.rC = W.rC; A.Tex = W.Tex; A.prf0 = W.prf0; A.rfy = W.rfy;
+    A.ph = W.ph; A.wN = wN; A.kx = W.kx; A.ky = W.ky; A.kz = W.kz; A.PC = W.PC; A.iPC = W.iPC; A.F0 = W.F0; A.F = W.F;
+    A.terms = W.terms; A.T0 = W.T0; A.rCt = W.tt; A.tt = W.tt; A.prf0 = W.prf0; A.rfy = W.rfy;
     double* cur = X;
     double* nxt = W.X2;
     DyrelCheck C;
@@ -714,10 +854,8 @@ int dim_dyrel(ht3d_ctx* ctx, double* X, DimWork& W, const double* wN, DimScal s,
         const bool storef = !chk && (iter == prm->nitmax || is_check(iter + 1, prm->nitout));
         s.h1 = S.h1; s.h2 = S.h2; s.dtau = S.dtau;
         A.Xin = cur; A.Xout = nxt;
-        if (chk) HT3D_LAUNCH(ctx, (k_dim_iter<PRESSURE, MODE_CHECK>), grd, blk, 0, A, s, b, nx, ny, nz);
-        else if (storef) HT3D_LAUNCH(ctx, (k_dim_iter<PRESSURE, MODE_STOREF>), grd, blk, 0, A, s, b, nx, ny, nz);
-        else HT3D_LAUNCH(ctx, (k_dim_iter<PRESSURE, MODE_PLAIN>), grd, blk, 0, A, s, b, nx, ny, nz);
-        HT3D_LAUNCH(ctx, k_dim_shell<PRESSURE>, sg, sb, 0, nxt, cur, W.ph, wN, W.ky, b, nx, ny, nz);
+        launch_after(ctx, pick(chk ? MODE_CHECK : (storef ? MODE_STOREF : MODE_PLAIN)), grd, L.threads, 0, A, s, b, nx,
+                     ny, nz, L.zchunk, wb, cb);
         std::swap(cur, nxt);
         it_done = iter;
         if (chk) {
@@ -766,6 +904,8 @@ extern "C" int ht3d_step_v18(ht3d_ctx* ctx, double* Tc_ex, double* Pc_ex, const 
         W.rfy = (double*)ht3d_scratch(ctx, SLOT_STEP_TY, sizeof(double) * nfy);
         W.terms = (double*)ht3d_scratch(ctx, SLOT_PARTIALS, sizeof(double) * (3 * n + 6 * ((n + 1023) / 1024 + 1)));
         W.ph = (signed char*)ht3d_scratch(ctx, SLOT_AUX2, nex);
+        W.iPC = (double*)ht3d_scratch(ctx, SLOT_AUX3, sizeof(double) * (1 + kRhofTerms) * n);
+        W.tt = W.iPC + n;
         const double dx = p->dx, dy = p->dy, dz = p->dz, _dx = 1.0 / dx, _dy = 1.0 / dy, _dz = 1.0 / dz;
         const double dt = p->dt, _dt = 1.0 / dt, transient = p->it == 0 ? 0.0 : 1.0;
         const dim3 gv = grid3(nx + 1, ny + 1, nz + 1, kBlock3), gc = grid3(nx, ny, nz, kBlock3);
