@@ -1,6 +1,7 @@
 // exp(x) and 10^x in IEEE double, identical bits on the host (g++,
 // -ffp-contract=off) and on the device (nvcc -fmad=false): only +, -, *, rint
-// and exact power-of-two scalings, each rounded as written.  The material
+// and exact power-of-two scalings, each rounded as written (on the device with
+// fewer operations on the FP64 pipe and the same results).  The material
 // laws of the dimensional model (fluid viscosity 10^(247.8/(T-140)) and
 // permeability exp(y/delta)) call these instead of the platform's libm or
 // CUDA's exp/exp10, whose last bits differ between machines, so the device
@@ -87,12 +88,43 @@ HT3D_EXPO_FN double ht3d_expo_finish(int N, double p) {
     const double s_hi = ht3d_expo_hi_host[j], s_lo = ht3d_expo_lo_host[j];
 #endif
     const double q = s_hi + (s_lo + (s_hi + s_lo) * p);  // q in [0.98, 2.03)
+#if defined(__CUDA_ARCH__)
+    // the exact scaling by 2^m on the exponent field: an integer addition instead of an FP64 product
+    if (m >= -1020 && m <= 1022) return __hiloint2double(__double2hiint(q) + (m << 20), __double2loint(q));
+#endif
     if (m > 1023) return q * ht3d_expo_from_bits((uint64_t)(m - 1 + 1023) << 52) * 2.0;
     if (m < -1021) return q * ht3d_expo_from_bits((uint64_t)(m + 54 + 1023) << 52) * 0x1p-54;
     return q * ht3d_expo_from_bits((uint64_t)(m + 1023) << 52);
 }
 
+// The reductions' integer N = rint(p), as an integer and as a double (|p| < 2^21).
+HT3D_EXPO_FN double ht3d_expo_round(double p, int* N) {
+#if defined(__CUDA_ARCH__)
+    // Adding 1.5 2^52 rounds to an integer (to even, as rint does) in the low
+    // word: two additions instead of a rounding and a conversion on the FP64 pipe.
+    const double t = p + 0x1.8p52;
+    *N = __double2loint(t);
+    return t - 0x1.8p52;
+#else
+    const double r = rint(p);
+    *N = (int)r;
+    return r;
+#endif
+}
+// NaN or beyond +-limit (|x| >= limit), on the device by integer compares
+HT3D_EXPO_FN int ht3d_expo_outside(double x, double limit) {
+#if defined(__CUDA_ARCH__)
+    return (__double_as_longlong(x) & 0x7fffffffffffffffLL) >= __double_as_longlong(limit);
+#else
+    return !(x > -limit && x < limit);
+#endif
+}
+
 // e^r - 1 for |r| <= ln2/64 (Taylor, degree 6, Horner)
+HT3D_EXPO_FN double ht3d_expo_poly1(double r) {  // ht3d_expo_poly(r, 0)
+    const double q = r * r * (HT3D_EXPO_A2 + r * (HT3D_EXPO_A3 + r * (HT3D_EXPO_A4 + r * (HT3D_EXPO_A5 + r * HT3D_EXPO_A6))));
+    return r + q;
+}
 HT3D_EXPO_FN double ht3d_expo_poly(double r1, double r2) {
     const double r = r1 + r2;
     const double q = r * r * (HT3D_EXPO_A2 + r * (HT3D_EXPO_A3 + r * (HT3D_EXPO_A4 + r * (HT3D_EXPO_A5 + r * HT3D_EXPO_A6))));
@@ -101,22 +133,36 @@ HT3D_EXPO_FN double ht3d_expo_poly(double r1, double r2) {
 
 // e^x
 HT3D_EXPO_FN double ht3d_exp(double x) {
-    if (x != x) return x + x;
-    if (x > 709.79) return ht3d_expo_from_bits(0x7ff0000000000000ull);
-    if (x < -745.2) return 0.0;
-    const double Nd = rint(x * HT3D_EXPO_INV_L);
+    if (ht3d_expo_outside(x, 709.0)) {
+        if (x != x) return x + x;
+        if (x > 709.79) return ht3d_expo_from_bits(0x7ff0000000000000ull);
+        if (x < -745.2) return 0.0;
+    }
+    int N;
+    const double Nd = ht3d_expo_round(x * HT3D_EXPO_INV_L, &N);
+#if defined(__CUDA_ARCH__)
+    const double r1 = __fma_rn(-Nd, HT3D_EXPO_L1, x);  // the product is exact
+#else
     const double r1 = x - Nd * HT3D_EXPO_L1;  // exact
+#endif
     const double r2 = -(Nd * HT3D_EXPO_L2);
-    return ht3d_expo_finish((int)Nd, ht3d_expo_poly(r1, r2));
+    return ht3d_expo_finish(N, ht3d_expo_poly(r1, r2));
 }
 
 // 10^x
 HT3D_EXPO_FN double ht3d_exp10(double x) {
-    if (x != x) return x + x;
-    if (x > 308.26) return ht3d_expo_from_bits(0x7ff0000000000000ull);
-    if (x < -323.62) return 0.0;
-    const double Nd = rint(x * HT3D_EXPO_INV_L10);
+    if (ht3d_expo_outside(x, 308.0)) {
+        if (x != x) return x + x;
+        if (x > 308.26) return ht3d_expo_from_bits(0x7ff0000000000000ull);
+        if (x < -323.62) return 0.0;
+    }
+    int N;
+    const double Nd = ht3d_expo_round(x * HT3D_EXPO_INV_L10, &N);
+#if defined(__CUDA_ARCH__)
+    const double r = __fma_rn(-Nd, HT3D_EXPO_L10_1, x) - Nd * HT3D_EXPO_L10_2;  // the first product is exact
+#else
     const double r = (x - Nd * HT3D_EXPO_L10_1) - Nd * HT3D_EXPO_L10_2;  // |r| <= log10(2)/64
+#endif
     const double s = r * HT3D_EXPO_LN10;                                   // |s| <= ln2/64
-    return ht3d_expo_finish((int)Nd, ht3d_expo_poly(s, 0.0));
+    return ht3d_expo_finish(N, ht3d_expo_poly1(s));
 }

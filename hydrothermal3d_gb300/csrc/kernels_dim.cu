@@ -19,13 +19,13 @@ namespace {
 // 8-point average of an extended centre field at vertex (i,j,k)
 // (Dimensional/kernels_HT3D_dimensional.jl:43-45)
 __device__ __forceinline__ double vtx8(const double* __restrict__ A, int i, int j, int k, int nx, int ny) {
-    double v = 1.0 / 8.0 * (A[EXI(i + 1, j + 1, k + 1)] + A[EXI(i + 1, j, k + 1)] + A[EXI(i, j + 1, k + 1)] + A[EXI(i, j, k + 1)]);
-    v += 1.0 / 8.0 * (A[EXI(i + 1, j + 1, k + 0)] + A[EXI(i + 1, j, k + 0)] + A[EXI(i, j + 1, k + 0)] + A[EXI(i, j, k + 0)]);
-    return v;
+    const double v = 1.0 / 8.0 * (A[EXI(i + 1, j + 1, k + 1)] + A[EXI(i + 1, j, k + 1)] + A[EXI(i, j + 1, k + 1)] + A[EXI(i, j, k + 1)]);
+    // v + 1/8 (...): the product is exact
+    return __fma_rn(1.0 / 8.0, A[EXI(i + 1, j + 1, k + 0)] + A[EXI(i + 1, j, k + 0)] + A[EXI(i, j + 1, k + 0)] + A[EXI(i, j, k + 0)], v);
 }
 
 __global__ void k_thermal_conductivity(double* ktv, const double* __restrict__ Tce, const double* __restrict__ phv,
-                                       double phi0, double scale_kt, double scale_T, int nx, int ny, int nz) {
+                                       double phi0, Divisor scale_kt, double scale_T, int nx, int ny, int nz) {
     GIDX;
     if (i > nx || j > ny || k > nz) return;
     double Tv = vtx8(Tce, i, j, k, nx, ny);
@@ -34,32 +34,47 @@ __global__ void k_thermal_conductivity(double* ktv, const double* __restrict__ T
     ktv[VXI(i, j, k)] = ((1 - law_phi(ph, phi0)) * law_kTs(Tv) + law_phi(ph, phi0) * law_kTf(Tv)) / scale_kt;
 }
 
+// kF depends on the row alone: the block's eight rows evaluate it once each (an
+// FP64 exponential costs the same issue slots whatever the number of active
+// lanes).  denom: the mode's divisor, scale_t, L^2/eta or L^2.
 __global__ void k_hydro_conductivity(double* kfv, const double* __restrict__ Tce, const double* __restrict__ Pce,
                                      const double* __restrict__ phv, double ymin, double dy, double k_fact, double delta,
-                                     double sc_s, double sc_T, double sc_L, double sc_t, double sc_eta, int mode,
+                                     double sc_s, double sc_T, double sc_L, Divisor denom, int mode,
                                      const double* __restrict__ kmul, int nx, int ny, int nz) {
     GIDX;
+    __shared__ double kF_row[8];
+    if (threadIdx.y == 0 && threadIdx.x < 8) {
+        const double y = ymin + (double)(blockIdx.y * 8 + threadIdx.x) * dy;
+        kF_row[threadIdx.x] = law_kF(y * sc_L, delta * sc_L);
+    }
+    __syncthreads();
     if (i > nx || j > ny || k > nz) return;
     double Tv = vtx8(Tce, i, j, k, nx, ny);
     Tv *= sc_T;
     if (Tv < 293.15) Tv = 293.15;
-    double Pv = vtx8(Pce, i, j, k, nx, ny);
-    Pv *= sc_s;
-    const double y = ymin + (double)j * dy;
-    double kF = law_kF(y * sc_L, delta * sc_L);
-    if (kmul) kF *= kmul[VXI(i, j, k)];
     const int v = VXI(i, j, k);
-    const double rk_mu = law_rhof_C(Tv - 273.15, Pv) * kF / law_muf(Tv);
-    double out = kfv[v];
-    if (mode == 1) out = rk_mu / sc_t;
-    else if (mode == 2) out = (kF / law_muf(Tv)) / (sc_L * sc_L / sc_eta);
-    else if (mode == 3) out = kF / (sc_L * sc_L);
+    double kF = kF_row[threadIdx.y];
+    if (kmul) kF *= kmul[v];
+    double out;
+    if (mode == 1) {
+        double Pv = vtx8(Pce, i, j, k, nx, ny);
+        Pv *= sc_s;
+        out = div_any(law_rhof_C(Tv - 273.15, Pv) * kF, law_muf(Tv)) / denom;
+    } else if (mode == 2) {
+        out = div_any(kF, law_muf(Tv)) / denom;
+    } else {
+        out = kF / denom;
+    }
     if (ph_eq(phv[v], 2.0)) out *= k_fact;
     kfv[v] = out;
 }
+// the divisor of a mode's permeability, as the reference forms it
+static Divisor hydro_denom(int mode, double sc_L, double sc_t, double sc_eta) {
+    return Divisor(mode == 1 ? sc_t : (mode == 2 ? sc_L * sc_L / sc_eta : sc_L * sc_L));
+}
 
 __global__ void k_fluid_density(double* rfv, const double* __restrict__ Tce, const double* __restrict__ Pce,
-                                const double* __restrict__ phv, double sc_s, double sc_T, double sc_rho, int nx, int ny,
+                                const double* __restrict__ phv, double sc_s, double sc_T, Divisor sc_rho, int nx, int ny,
                                 int nz) {
     GIDX;
     if (i > nx || j > ny || k > nz) return;
@@ -69,7 +84,7 @@ __global__ void k_fluid_density(double* rfv, const double* __restrict__ Tce, con
     Pv *= sc_s;
     const int v = VXI(i, j, k);
     double r = law_rhof_C(Tv - 273.15, Pv) / sc_rho;
-    if (ph_eq(phv[v], 1.0)) r = 0.000 / sc_rho;
+    if (ph_eq(phv[v], 1.0)) r = 0.000 / sc_rho.b;
     rfv[v] = r;
 }
 
@@ -102,7 +117,7 @@ __global__ void k_init_conductivity(double* kx, double* ky, double* kz, const do
 }
 // ComputeρCeffective!  :148-160
 __global__ void k_rhoC_eff(double* rC, const double* __restrict__ T, const double* __restrict__ P,
-                           const double* __restrict__ phc, double phii, double sT, double ss, double sC, double srho,
+                           const double* __restrict__ phc, double phii, double sT, double ss, Divisor sC, Divisor srho,
                            int nx, int ny, int nz) {
     GIDX;
     if (i >= nx || j >= ny || k >= nz) return;
@@ -134,8 +149,7 @@ __global__ void k_res_temperature(double* F, const double* __restrict__ T, const
         f += (qy[ix3(i, j + 1, k, nx, ny + 1)] - qy[ix3(i, j, k, nx, ny + 1)]) * _dy;
         f += (qz[ix3(i, j, k + 1, nx, ny)] - qz[ix3(i, j, k, nx, ny)]) * _dz;
         f -= transient * Q;
-        f /= PC[c];
-        F[c] = f;
+        F[c] = div_any(f, PC[c]);
     } else {
         F[c] = 0.;
     }
@@ -196,7 +210,7 @@ __global__ void k_dim_bcs(double* X, double* B, const double* __restrict__ ky, c
 }
 // ϕρf (:225-235), ϕρf_old (:237-247, cell inputs), ϕdρdP! (:249-259)
 __global__ void k_phi_rhof(double* out, const double* __restrict__ T, const double* __restrict__ P,
-                           const double* __restrict__ phc, double phii, double srho, double sT, double ss, int cell_in,
+                           const double* __restrict__ phc, double phii, Divisor denom, double sT, double ss, int cell_in,
                            int deriv, int nx, int ny, int nz) {
     GIDX;
     if (i >= nx || j >= ny || k >= nz) return;
@@ -205,8 +219,8 @@ __global__ void k_phi_rhof(double* out, const double* __restrict__ T, const doub
         const int s = cell_in ? CI(i, j, k) : EXI(i + 1, j + 1, k + 1);
         const double Tc = T[s] * sT - 273.15;
         const double Pc = P[s] * ss;
-        out[CI(i, j, k)] = deriv ? law_phi(ph, phii) * law_drhodP_C(Tc, Pc) / (srho / ss)
-                                 : law_phi(ph, phii) * law_rhof_C(Tc, Pc) / srho;
+        // denom: scale_rho, or scale_rho / scale_sigma for the derivative
+        out[CI(i, j, k)] = (deriv ? law_phi(ph, phii) * law_drhodP_C(Tc, Pc) : law_phi(ph, phii) * law_rhof_C(Tc, Pc)) / denom;
     }
 }
 // ComputeDarcyFlux!  :266-272
@@ -244,8 +258,7 @@ __global__ void k_res_pressure(double* F, const double* __restrict__ phc, const 
         f += (qx[ix3(i + 1, j, k, nx + 1, ny)] - qx[ix3(i, j, k, nx + 1, ny)]) * _dx;
         f += (qy[ix3(i, j + 1, k, nx, ny + 1)] - qy[ix3(i, j, k, nx, ny + 1)]) * _dy;
         f += (qz[ix3(i, j, k + 1, nx, ny)] - qz[ix3(i, j, k, nx, ny)]) * _dz;
-        f /= PC[c];
-        F[c] = f;
+        F[c] = div_any(f, PC[c]);
     } else {
         F[c] = 0.;
     }
@@ -257,15 +270,15 @@ __global__ void k_init_vel_dim(double* Vx, double* Vy, double* Vz, const double*
     GIDX;
     if (i < nx + 1 && j < ny && k < nz) {
         const int f = ix3(i, j, k, nx + 1, ny);
-        Vx[f] = qx[f] / ((rfv[VXI(i, j, k)] + rfv[VXI(i, j + 1, k)] + rfv[VXI(i, j, k + 1)] + rfv[VXI(i, j + 1, k + 1)]) * 0.25);
+        Vx[f] = div_any(qx[f], ((rfv[VXI(i, j, k)] + rfv[VXI(i, j + 1, k)] + rfv[VXI(i, j, k + 1)] + rfv[VXI(i, j + 1, k + 1)]) * 0.25));
     }
     if (i < nx && j < ny + 1 && k < nz) {
         const int f = ix3(i, j, k, nx, ny + 1);
-        Vy[f] = qy[f] / ((rfv[VXI(i, j, k)] + rfv[VXI(i + 1, j, k)] + rfv[VXI(i, j, k + 1)] + rfv[VXI(i + 1, j, k + 1)]) * 0.25);
+        Vy[f] = div_any(qy[f], ((rfv[VXI(i, j, k)] + rfv[VXI(i + 1, j, k)] + rfv[VXI(i, j, k + 1)] + rfv[VXI(i + 1, j, k + 1)]) * 0.25));
     }
     if (i < nx && j < ny && k < nz + 1) {
         const int f = ix3(i, j, k, nx, ny);
-        Vz[f] = qz[f] / ((rfv[VXI(i, j, k)] + rfv[VXI(i + 1, j, k)] + rfv[VXI(i, j + 1, k)] + rfv[VXI(i + 1, j + 1, k)]) * 0.25);
+        Vz[f] = div_any(qz[f], ((rfv[VXI(i, j, k)] + rfv[VXI(i + 1, j, k)] + rfv[VXI(i, j + 1, k)] + rfv[VXI(i + 1, j + 1, k)]) * 0.25));
     }
 }
 __global__ void k_law_eval(double* out, const double* __restrict__ a, const double* __restrict__ b, int which, long long n) {
@@ -285,7 +298,7 @@ int ht3d_ComputeThermalConductivity(ht3d_ctx* ctx, double* ktv, const double* Tc
     return ht3d_guard(ctx, [&]() {
         HT3D_REQUIRE(all_nonnull(ktv, Tce, phv), "null argument");
         DIMS;
-        HT3D_LAUNCH(ctx, k_thermal_conductivity, G3(nx + 1, ny + 1, nz + 1), kBlock3, 0, ktv, Tce, phv, phi0, scale_kt,
+        HT3D_LAUNCH(ctx, k_thermal_conductivity, G3(nx + 1, ny + 1, nz + 1), kBlock3, 0, ktv, Tce, phv, phi0, Divisor(scale_kt),
                     scale_T, nx, ny, nz);
         return HT3D_OK;
     });
@@ -300,7 +313,8 @@ int ht3d_ComputeHydroConductivity(ht3d_ctx* ctx, double* kfv, const double* Tce,
         DIMS;
         HT3D_REQUIRE(mode >= 1 && mode <= 3, "mode must be 1, 2 or 3");
         HT3D_LAUNCH(ctx, k_hydro_conductivity, G3(nx + 1, ny + 1, nz + 1), kBlock3, 0, kfv, Tce, Pce, phv, ymin, dy,
-                    k_fact, delta, scale_sigma, scale_T, scale_L, scale_t, scale_eta, mode, kmul_v, nx, ny, nz);
+                    k_fact, delta, scale_sigma, scale_T, scale_L, hydro_denom(mode, scale_L, scale_t, scale_eta), mode,
+                    kmul_v, nx, ny, nz);
         return HT3D_OK;
     });
 }
@@ -311,7 +325,7 @@ int ht3d_ComputeFluidDensity(ht3d_ctx* ctx, double* rhofv, const double* Tce, co
         HT3D_REQUIRE(all_nonnull(rhofv, Tce, Pce, phv), "null argument");
         DIMS;
         HT3D_LAUNCH(ctx, k_fluid_density, G3(nx + 1, ny + 1, nz + 1), kBlock3, 0, rhofv, Tce, Pce, phv, scale_sigma,
-                    scale_T, scale_rho, nx, ny, nz);
+                    scale_T, Divisor(scale_rho), nx, ny, nz);
         return HT3D_OK;
     });
 }
@@ -351,7 +365,7 @@ int ht3d_ComputeRhoCeffective(ht3d_ctx* ctx, double* rhoC_eff, const double* Tc_
         HT3D_REQUIRE(all_nonnull(rhoC_eff, Tc_ex, Pc_ex, phc_ex), "null argument");
         DIMS;
         HT3D_LAUNCH(ctx, k_rhoC_eff, G3(nx, ny, nz), kBlock3, 0, rhoC_eff, Tc_ex, Pc_ex, phc_ex, phi_i, sca_T, sca_sigma,
-                    sca_C, sca_rho, nx, ny, nz);
+                    Divisor(sca_C), Divisor(sca_rho), nx, ny, nz);
         return HT3D_OK;
     });
 }
@@ -408,8 +422,8 @@ int ht3d_PhiRhof(ht3d_ctx* ctx, double* phirhofc, const double* Tc_ex, const dou
     return ht3d_guard(ctx, [&]() {
         HT3D_REQUIRE(all_nonnull(phirhofc, Tc_ex, Pc_ex, phc_ex), "null argument");
         DIMS;
-        HT3D_LAUNCH(ctx, k_phi_rhof, G3(nx, ny, nz), kBlock3, 0, phirhofc, Tc_ex, Pc_ex, phc_ex, phi_i, scale_rho,
-                    scale_T, scale_sigma, 0, 0, nx, ny, nz);
+        HT3D_LAUNCH(ctx, k_phi_rhof, G3(nx, ny, nz), kBlock3, 0, phirhofc, Tc_ex, Pc_ex, phc_ex, phi_i,
+                    Divisor(scale_rho), scale_T, scale_sigma, 0, 0, nx, ny, nz);
         return HT3D_OK;
     });
 }
@@ -419,8 +433,8 @@ int ht3d_PhiRhofOld(ht3d_ctx* ctx, double* phirhofc, const double* Tc0, const do
     return ht3d_guard(ctx, [&]() {
         HT3D_REQUIRE(all_nonnull(phirhofc, Tc0, Pc0, phc_ex), "null argument");
         DIMS;
-        HT3D_LAUNCH(ctx, k_phi_rhof, G3(nx, ny, nz), kBlock3, 0, phirhofc, Tc0, Pc0, phc_ex, phi_i, scale_rho, scale_T,
-                    scale_sigma, 1, 0, nx, ny, nz);
+        HT3D_LAUNCH(ctx, k_phi_rhof, G3(nx, ny, nz), kBlock3, 0, phirhofc, Tc0, Pc0, phc_ex, phi_i, Divisor(scale_rho),
+                    scale_T, scale_sigma, 1, 0, nx, ny, nz);
         return HT3D_OK;
     });
 }
@@ -430,8 +444,8 @@ int ht3d_PhiDrhodP(ht3d_ctx* ctx, double* phidrhodP, const double* Tc_ex, const 
     return ht3d_guard(ctx, [&]() {
         HT3D_REQUIRE(all_nonnull(phidrhodP, Tc_ex, Pc_ex, phc_ex), "null argument");
         DIMS;
-        HT3D_LAUNCH(ctx, k_phi_rhof, G3(nx, ny, nz), kBlock3, 0, phidrhodP, Tc_ex, Pc_ex, phc_ex, phi_i, scale_rho,
-                    scale_T, scale_sigma, 0, 1, nx, ny, nz);
+        HT3D_LAUNCH(ctx, k_phi_rhof, G3(nx, ny, nz), kBlock3, 0, phidrhodP, Tc_ex, Pc_ex, phc_ex, phi_i,
+                    Divisor(scale_rho / scale_sigma), scale_T, scale_sigma, 0, 1, nx, ny, nz);
         return HT3D_OK;
     });
 }
@@ -758,18 +772,16 @@ __global__ void k_inn_copy(double* A, const double* __restrict__ B, int nx, int 
     for_cells_z(nx, ny, nz, [&](int i, int j, int k) { A[CI(i, j, k)] = B[EXI(i + 1, j + 1, k + 1)]; });
 }
 __global__ void k_gersh(double* G, double* D, const double* __restrict__ rC, const double* __restrict__ kx,
-                        const double* __restrict__ ky, const double* __restrict__ kz, double transient, double dt,
-                        double dx, double dy, double dz, int nx, int ny, int nz) {
+                        const double* __restrict__ ky, const double* __restrict__ kz, double transient, GershSpacing h,
+                        int nx, int ny, int nz) {
     GIDX;
     if (i >= nx || j >= ny || k >= nz) return;
-    const double kW = kx[ix3(i, j, k, nx + 1, ny)], kE = kx[ix3(i + 1, j, k, nx + 1, ny)];
-    const double kS = ky[ix3(i, j, k, nx, ny + 1)], kN = ky[ix3(i, j + 1, k, nx, ny + 1)];
-    const double kB = kz[CI(i, j, k)], kF = kz[CI(i, j, k + 1)], rhoC = rC[CI(i, j, k)];
-    const double diag = ((kB / dz + kF / dz) / dz + (kN / dy + kS / dy) / dy + (kE / dx + kW / dx) / dx + rhoC * transient / dt);
-    double g = fabs(kE / (dx * dx)) + fabs(kW / (dx * dx)) + fabs(kN / (dy * dy)) + fabs(kS / (dy * dy)) +
-               fabs(kB / (dz * dz)) + fabs(kF / (dz * dz)) + fabs(diag);
+    double diag;
+    const double g = gershgorin_row(kx[ix3(i, j, k, nx + 1, ny)], kx[ix3(i + 1, j, k, nx + 1, ny)],
+                                    ky[ix3(i, j, k, nx, ny + 1)], ky[ix3(i, j + 1, k, nx, ny + 1)], kz[CI(i, j, k)],
+                                    kz[CI(i, j, k + 1)], rC[CI(i, j, k)], transient, h, diag);
     D[CI(i, j, k)] = diag;
-    G[CI(i, j, k)] = g / diag;
+    G[CI(i, j, k)] = div_any(g, diag);
 }
 
 // blocks of `threads` that cover the ghost shell (edges twice)
@@ -925,13 +937,13 @@ extern "C" int ht3d_step_v18(ht3d_ctx* ctx, double* Tc_ex, double* Pc_ex, const 
         };
         int st = HT3D_OK;
         if (p->thermal) {
-            HT3D_LAUNCH(ctx, k_thermal_conductivity, gv, kBlock3, 0, W.kv, Tc_ex, phv, p->phi_i, p->sc_kt, p->sc_T, nx,
+            HT3D_LAUNCH(ctx, k_thermal_conductivity, gv, kBlock3, 0, W.kv, Tc_ex, phv, p->phi_i, Divisor(p->sc_kt), p->sc_T, nx,
                         ny, nz);
             smooth();
             HT3D_LAUNCH(ctx, k_rhoC_eff, gc, kBlock3, 0, W.rC, Tc_ex, Pc_ex, phc_ex, p->phi_i, p->sc_T, p->sc_sigma,
-                        p->sc_C, p->sc_rho, nx, ny, nz);
-            HT3D_LAUNCH(ctx, k_gersh, gc, kBlock3, 0, W.G, W.PC, W.rC, W.kx, W.ky, W.kz, transient, dt, dx, dy, dz, nx,
-                        ny, nz);
+                        Divisor(p->sc_C), Divisor(p->sc_rho), nx, ny, nz);
+            HT3D_LAUNCH(ctx, k_gersh, gc, kBlock3, 0, W.G, W.PC, W.rC, W.kx, W.ky, W.kz, transient,
+                        GershSpacing(dt, dx, dy, dz), nx, ny, nz);
             DimBC b{p->Ttop, p->qyS / _dy, _dy};
             const double lmax = ht3d_reduce_device(ctx, W.G, n, RED_MAX, nullptr);
             st = dim_dyrel<0>(ctx, Tc_ex, W, wN, s, b, lmax, &p->thermal_dyrel, st_T, nx, ny, nz);
@@ -939,18 +951,19 @@ extern "C" int ht3d_step_v18(ht3d_ctx* ctx, double* Tc_ex, double* Pc_ex, const 
         }
         if (p->hydro) {
             HT3D_LAUNCH(ctx, k_hydro_conductivity, gv, kBlock3, 0, W.kv, Tc_ex, Pc_ex, phv, p->ymin, dy, p->k_fact,
-                        p->delta, p->sc_sigma, p->sc_T, p->sc_L, p->sc_t, p->sc_eta, 1, kmul_v, nx, ny, nz);
+                        p->delta, p->sc_sigma, p->sc_T, p->sc_L, hydro_denom(1, p->sc_L, p->sc_t, p->sc_eta), 1, kmul_v, nx, ny,
+                        nz);
             smooth();
-            HT3D_LAUNCH(ctx, k_phi_rhof, gc, kBlock3, 0, W.rC, Tc_ex, Pc_ex, phc_ex, p->phi_i, p->sc_rho, p->sc_T,
-                        p->sc_sigma, 0, 1, nx, ny, nz);
-            HT3D_LAUNCH(ctx, k_gersh, gc, kBlock3, 0, W.G, W.PC, W.rC, W.kx, W.ky, W.kz, transient, dt, dx, dy, dz, nx,
-                        ny, nz);
+            HT3D_LAUNCH(ctx, k_phi_rhof, gc, kBlock3, 0, W.rC, Tc_ex, Pc_ex, phc_ex, p->phi_i,
+                        Divisor(p->sc_rho / p->sc_sigma), p->sc_T, p->sc_sigma, 0, 1, nx, ny, nz);
+            HT3D_LAUNCH(ctx, k_gersh, gc, kBlock3, 0, W.G, W.PC, W.rC, W.kx, W.ky, W.kz, transient,
+                        GershSpacing(dt, dx, dy, dz), nx, ny, nz);
             const double lmax = ht3d_reduce_device(ctx, W.G, n, RED_MAX, nullptr);
             // the reference reuses the Gershgorin array (Xc0) for ϕρf_old (v18:500)
-            HT3D_LAUNCH(ctx, k_phi_rhof, gc, kBlock3, 0, W.G, W.T0, W.P0, phc_ex, p->phi_i, p->sc_rho, p->sc_T,
-                        p->sc_sigma, 1, 0, nx, ny, nz);
+            HT3D_LAUNCH(ctx, k_phi_rhof, gc, kBlock3, 0, W.G, W.T0, W.P0, phc_ex, p->phi_i, Divisor(p->sc_rho),
+                        p->sc_T, p->sc_sigma, 1, 0, nx, ny, nz);
             W.prf0 = W.G;
-            HT3D_LAUNCH(ctx, k_fluid_density, gv, kBlock3, 0, W.kv, Tc_ex, Pc_ex, phv, p->sc_sigma, p->sc_T, p->sc_rho,
+            HT3D_LAUNCH(ctx, k_fluid_density, gv, kBlock3, 0, W.kv, Tc_ex, Pc_ex, phv, p->sc_sigma, p->sc_T, Divisor(p->sc_rho),
                         nx, ny, nz);
             HT3D_LAUNCH(ctx, k_av_xza, grid3(nx, ny + 1, nz, kBlock3), kBlock3, 0, W.rfy, W.kv, nx, ny, nz);
             DimBC b{p->Ptop, 0.0, _dy};
@@ -959,9 +972,9 @@ extern "C" int ht3d_step_v18(ht3d_ctx* ctx, double* Tc_ex, double* Pc_ex, const 
         }
         // velocity (v18:543-548)
         HT3D_LAUNCH(ctx, k_hydro_conductivity, gv, kBlock3, 0, W.kv, Tc_ex, Pc_ex, phv, p->ymin, dy, p->k_fact, p->delta,
-                    p->sc_sigma, p->sc_T, p->sc_L, p->sc_t, p->sc_eta, 2, kmul_v, nx, ny, nz);
+                    p->sc_sigma, p->sc_T, p->sc_L, hydro_denom(2, p->sc_L, p->sc_t, p->sc_eta), 2, kmul_v, nx, ny, nz);
         smooth();
-        HT3D_LAUNCH(ctx, k_fluid_density, gv, kBlock3, 0, W.kv, Tc_ex, Pc_ex, phv, p->sc_sigma, p->sc_T, p->sc_rho, nx,
+        HT3D_LAUNCH(ctx, k_fluid_density, gv, kBlock3, 0, W.kv, Tc_ex, Pc_ex, phv, p->sc_sigma, p->sc_T, Divisor(p->sc_rho), nx,
                     ny, nz);
         HT3D_LAUNCH(ctx, k_darcy_flux, gv, kBlock3, 0, Vx, Vy, Vz, W.kv, W.kx, W.ky, W.kz, Pc_ex, p->g, _dx, _dy, _dz,
                     nx, ny, nz);

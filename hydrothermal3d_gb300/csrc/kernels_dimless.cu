@@ -9,6 +9,7 @@
 // granular, reference-shaped entry points; the fused solver in dyrel.cu is the
 // fast path.
 #include "ht3d_internal.cuh"
+#include "fp64_div.cuh"
 
 #define GIDX                                                \
     const int i = blockIdx.x * blockDim.x + threadIdx.x;    \
@@ -211,21 +212,19 @@ __global__ void k_cpy_inn(double* A, const double* __restrict__ B, int nx, int n
 // (HYDRO = 1: GershgorinHydro! :335-347, G only, no division)
 template <int HYDRO>
 __global__ void k_gershgorin(double* G, double* D, const double* __restrict__ rC, const double* __restrict__ kx,
-                             const double* __restrict__ ky, const double* __restrict__ kz, double transient, double dt,
-                             double dx, double dy, double dz, int nx, int ny, int nz) {
+                             const double* __restrict__ ky, const double* __restrict__ kz, double transient,
+                             GershSpacing h, int nx, int ny, int nz) {
     GIDX;
     if (i >= nx || j >= ny || k >= nz) return;
-    const double kW = FX(kx, i, j, k), kE = FX(kx, i + 1, j, k), kS = FY(ky, i, j, k), kN = FY(ky, i, j + 1, k),
-                 kF = FZ(kz, i, j, k + 1), kB = FZ(kz, i, j, k), rhoC = CX(rC, i, j, k);
-    const double diag = ((kB / dz + kF / dz) / dz + (kN / dy + kS / dy) / dy + (kE / dx + kW / dx) / dx + rhoC * transient / dt);
-    double g = fabs(kE / (dx * dx)) + fabs(kW / (dx * dx)) + fabs(kN / (dy * dy)) + fabs(kS / (dy * dy)) +
-               fabs(kB / (dz * dz)) + fabs(kF / (dz * dz)) + fabs(diag);
+    double diag;
+    const double g = gershgorin_row(FX(kx, i, j, k), FX(kx, i + 1, j, k), FY(ky, i, j, k), FY(ky, i, j + 1, k),
+                                    FZ(kz, i, j, k), FZ(kz, i, j, k + 1), CX(rC, i, j, k), transient, h, diag);
     if (HYDRO) {
         CX(G, i, j, k) = g;
         return;
     }
     CX(D, i, j, k) = diag;
-    CX(G, i, j, k) = g / diag;
+    CX(G, i, j, k) = div_any(g, diag);
 }
 
 __global__ void k_swap_dyrel(double* Xc, double* Yc, const double* __restrict__ X0, const double* __restrict__ Y0,
@@ -453,8 +452,8 @@ int ht3d_GershgorinPoisson(ht3d_ctx* ctx, double* G, double* D, const double* rh
     return ht3d_guard(ctx, [&]() {
         HT3D_REQUIRE(all_nonnull(G, D, rhoC_eff, kx, ky, kz), "null argument");
         DIMS_OK(1);
-        HT3D_LAUNCH(ctx, k_gershgorin<0>, G3(nx, ny, nz), kBlock3, 0, G, D, rhoC_eff, kx, ky, kz, transient, dt, dx, dy,
-                    dz, nx, ny, nz);
+        HT3D_LAUNCH(ctx, k_gershgorin<0>, G3(nx, ny, nz), kBlock3, 0, G, D, rhoC_eff, kx, ky, kz, transient,
+                    GershSpacing(dt, dx, dy, dz), nx, ny, nz);
         return HT3D_OK;
     });
 }
@@ -466,7 +465,7 @@ int ht3d_GershgorinHydro(ht3d_ctx* ctx, double* G, const double* phidrhodP, cons
         HT3D_REQUIRE(all_nonnull(G, phidrhodP, kx, ky, kz), "null argument");
         DIMS_OK(1);
         HT3D_LAUNCH(ctx, k_gershgorin<1>, G3(nx, ny, nz), kBlock3, 0, G, (double*)nullptr, phidrhodP, kx, ky, kz,
-                    transient, dt, dx, dy, dz, nx, ny, nz);
+                    transient, GershSpacing(dt, dx, dy, dz), nx, ny, nz);
         return HT3D_OK;
     });
 }

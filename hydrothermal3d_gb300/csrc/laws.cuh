@@ -3,6 +3,8 @@
 // x^2 and x^3 are products as Julia's literal powers; x^4 is (x^2)^2.
 #pragma once
 #include "expo.h"
+#include "fp64_div.cuh"
+#include "ht3d_internal.cuh"
 
 __host__ __device__ inline double law_kTs(double T) { return 3.1138 - 0.0023 * (T); }
 __host__ __device__ inline double law_kTf(double T) { return -0.069 + 0.0012 * (T); }
@@ -22,9 +24,15 @@ __host__ __device__ inline double law_drhodP_C(double T_C, double p) {
 }
 // 10^x and e^x: ht3d_exp10/ht3d_exp (expo.h), one implementation whose bits
 // are the same on the device and in the host's CPU oracle
-__host__ __device__ inline double law_muf(double T) { return 2.414e-5 * ht3d_exp10(247.8 / (T - 140.)); }
+#if defined(__CUDA_ARCH__)
+__device__ inline double law_muf(double T) { return 2.414e-5 * ht3d_exp10(div_any(247.8, T - 140.)); }
+// the phase by its bits (ph_eq): no FP64 compare
+__device__ inline double law_phi(double phase, double phi0) { return ph_eq(phase, 2.0) ? 3 * phi0 : phi0; }
+#else
+__host__ inline double law_muf(double T) { return 2.414e-5 * ht3d_exp10(247.8 / (T - 140.)); }
+__host__ inline double law_phi(double phase, double phi0) { return phase == 2.0 ? 3 * phi0 : phi0; }
+#endif
 __host__ __device__ inline double law_kF(double y, double delta) { return 5e-16 * ht3d_exp(y / delta); }
-__host__ __device__ inline double law_phi(double phase, double phi0) { return phase == 2.0 ? 3 * phi0 : phi0; }
 
 // index: 0 kTs, 1 kTf, 2 Cf, 3 Cs, 4 rhos, 5 rhof_C(T_C,p), 6 drhodP_C(T_C,p), 7 muf, 8 kF(y,delta), 9 phi(phase,phi0),
 // 10 e^a, 11 10^a (the exponentials the laws use)

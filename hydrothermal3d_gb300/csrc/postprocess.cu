@@ -93,7 +93,7 @@ __global__ void k_post(PostOut o, PostIn a, ht3d_post_params p, const double* __
         if (o.Pe) {
             const double V = sqrt(vx * vx + vy * vy + vz * vz);
             const double C = law_Cf(T);
-            o.Pe[c] = p.scale_L * rho * C * V / keff;
+            o.Pe[c] = div_any(p.scale_L * rho * C * V, keff);
         }
     }
     if (o.Ceff) o.Ceff[c] = law_Cs(T);
