@@ -446,11 +446,25 @@ struct LineSrc {
     __device__ __forceinline__ void put(int c, T val) const { out[(long long)c * stride] = val; }
 };
 
-// Balanced segments: kMarchL cells per thread on average, at least 48 each
-// when a line has more than one.
-constexpr int kMarchL = 64;
 constexpr int kMarchUnroll = 4;  // steps per software-pipelined body of the y/z march
-__host__ __device__ __forceinline__ int march_chunks(int n) { return n < 3 * kMarchL / 2 ? 1 : (n + kMarchL / 2) / kMarchL; }
+constexpr int kMarchL = 64, kMarchMin = 8;
+constexpr long long kWarpsF32 = 1216, kWarpsMixed = 608;
+int long_segments(int n) { return n < 3 * kMarchL / 2 ? 1 : (n + kMarchL / 2) / kMarchL; }
+// Segments that the lines of a sweep are cut into, `warps` warps of lines: K
+// where the lines alone fill the chip (whole rows along x, which the sweep may
+// update in place: 511^3 2.54 ms, 3.15 with rows cut at 64 cells; 64 cells per
+// thread along y and z); shorter ones, down to 8
+// (a segment's first steps read six cells before it), until there are `want`
+// warps.  A segment begins with about five steps' work that its neighbour does
+// as well, so more warps than that are slower: FP32 1216 (127^3: 87 us; 97 with
+// four times as many), mixed, where one warp per scheduler fills the FP64 pipe,
+// 608 (95^3: 276 us; 404 with twice as many).  Sweep before (segments of 48 and
+// more) and now, FP32 and mixed: 33 x 29 x 31 53 -> 39 and 169 -> 83 us, 63^3 81 ->
+// 39 and 313 -> 136, 95^3 109 -> 58 and 463 -> 276.
+int march_segments(long long warps, int n, long long want, int K) {
+    while (warps * K < want && n / (K + 1) >= kMarchMin) ++K;
+    return K;
+}
 
 template <int AXIS, class Stream>
 __global__ void __launch_bounds__(128) k_weno_march(const typename Stream::value* __restrict__ src,
@@ -462,7 +476,7 @@ __global__ void __launch_bounds__(128) k_weno_march(const typename Stream::value
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int o = blockIdx.y;  // k for the y-march, j for the z-march
     const int n = AXIS == 1 ? ny : nz;
-    const int K = march_chunks(n);
+    const int K = gridDim.z;  // segments of a line (march_segments)
     const int c0 = (int)((long long)blockIdx.z * n / K), c1 = (int)((long long)(blockIdx.z + 1) * n / K);
     if (i >= nx) return;
     const int n1 = nx + 2, n2 = ny + 2;
@@ -562,14 +576,16 @@ struct RingSrc {
     __device__ __forceinline__ void put(int c, T val) const { t[col(c)] = val; }
 };
 
-// The x sweep updates T in place, so a row is never split between warps:
+// In place (dst == T) a row is never split between warps:
 // a segment's halo (six cells on each side) would be the neighbouring
 // segment's cells, which another block may already have overwritten.  Within
 // a warp the ring's copies run ahead of its stores (tile v + 4 is fetched
 // after tile v + 1 is stored), so whole rows are safe.
-template <class Stream>
+// WHOLE: whole rows, in place (T is not read); else segments, T -> dst.
+template <class Stream, bool WHOLE>
 __global__ void __launch_bounds__(32 * XWarps<typename Stream::value>::value)
-    k_weno_xstream(typename Stream::value* __restrict__ T, const typename Stream::value* __restrict__ Vx,
+    k_weno_xstream(const typename Stream::value* __restrict__ T, typename Stream::value* __restrict__ dst,
+                   const typename Stream::value* __restrict__ Vx,
                    typename Stream::value dt, typename Stream::param h, typename Stream::bc_type bc, int nx, int ny,
                    int nz) {
     using E = typename Stream::value;
@@ -580,7 +596,9 @@ __global__ void __launch_bounds__(32 * XWarps<typename Stream::value>::value)
     const long long row0 = ((long long)blockIdx.x * kXWarps + warp) * 32;
     if (row0 >= rows) return;  // whole warps only
     const int n = nx;
-    const int c0 = 0, c1 = n;  // whole rows (see above)
+    const int K = WHOLE ? 1 : gridDim.y;  // segments of a row
+    const int c0 = WHOLE ? 0 : (int)((long long)blockIdx.y * n / K);
+    const int c1 = WHOLE ? n : (int)((long long)(blockIdx.y + 1) * n / K);
     const int b0 = c0 - kXW;
     E* tr = ring[warp][0];
     E* vr = ring[warp][1];
@@ -600,7 +618,7 @@ __global__ void __launch_bounds__(32 * XWarps<typename Stream::value>::value)
             rel[k] = (unsigned)(tbase + (long long)(nx + 2) * (r + 2 * (r / ny)) - t0off);
         }
     }
-    const E* Tw = T + t0off;
+    const E* Tw = (WHOLE ? dst : T) + t0off;
     const E* Vw = Vx + (long long)(nx + 1) * row0;
     const int tq_lo = max(0, c0 - 6), tq_hi = min(n, c1 + 6);  // T0 positions a segment reads
     const int vq_lo = max(0, c0 - 3), vq_hi = min(n, c1 + 3);  // faces (inclusive)
@@ -625,7 +643,7 @@ __global__ void __launch_bounds__(32 * XWarps<typename Stream::value>::value)
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const int r = sub + 4 * k;
-            if (row0 + r <= rlast) T[t0off + rel[k] + q] = ts[r * kXPitch];
+            if (row0 + r <= rlast) dst[t0off + rel[k] + q] = ts[r * kXPitch];
         }
     };
     load_tile(0);
@@ -753,7 +771,8 @@ __global__ void __launch_bounds__(256) k_weno_stage_f32(const float* __restrict_
 }
 
 // inner cells of a ghosted field: dst = src
-__global__ void k_copy_inner_f32(float* __restrict__ dst, const float* __restrict__ src, int nx, int ny, int nz) {
+template <class T>
+__global__ void k_copy_inner(T* __restrict__ dst, const T* __restrict__ src, int nx, int ny, int nz) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int k = blockIdx.z;
@@ -777,9 +796,12 @@ float* axis_f32(ht3d_ctx* ctx, float* cur, float* other, float* tmp, const float
             using S = typename StreamOf<QUIRK>::type;
             constexpr int warps = XWarps<float>::value;
             const long long rows = (long long)ny * nz, per_block = 32LL * warps;
-            const dim3 g((unsigned)((rows + per_block - 1) / per_block));
-            HT3D_LAUNCH(ctx, k_weno_xstream<S>, g, 32 * warps, 0, cur, V, dt, h, bcf(bc), nx, ny, nz);
-            return cur;
+            const int K = march_segments((rows + 31) / 32, nx, kWarpsF32, 1);
+            float* to = K == 1 ? cur : other;  // in place only over whole rows
+            const dim3 g((unsigned)((rows + per_block - 1) / per_block), K);
+            if (K == 1) HT3D_LAUNCH(ctx, (k_weno_xstream<S, true>), g, 32 * warps, 0, cur, to, V, dt, h, bcf(bc), nx, ny, nz);
+            else HT3D_LAUNCH(ctx, (k_weno_xstream<S, false>), g, 32 * warps, 0, cur, to, V, dt, h, bcf(bc), nx, ny, nz);
+            return to;
         }
         const size_t smem = sizeof(float) * 2 * (size_t)(nx + 6) * kRowWarps;
         if (smem <= 96 * 1024) {
@@ -794,7 +816,8 @@ float* axis_f32(ht3d_ctx* ctx, float* cur, float* other, float* tmp, const float
     } else {
         if (!periodic) {
             const int n = AXIS == 1 ? ny : nz;
-            const dim3 g((nx + 127) / 128, AXIS == 1 ? nz : ny, march_chunks(n));
+            const dim3 g((nx + 127) / 128, AXIS == 1 ? nz : ny,
+                         march_segments((nx + 31) / 32 * (AXIS == 1 ? nz : ny), n, kWarpsF32, long_segments(n)));
             HT3D_LAUNCH(ctx, (k_weno_march<AXIS, typename StreamOf<QUIRK>::type>), g, 128, 0, cur, other, V, dt, h,
                         bcf(bc), nx, ny, nz);
             return other;
@@ -816,24 +839,35 @@ void all_f32(ht3d_ctx* ctx, float* T, float* S, float* tmp, const float* const* 
     cur = axis_f32<2, QUIRK>(ctx, cur, cur == T ? S : T, tmp, V[2], dt, h[2], bc[2], nx, ny, nz);
     if (cur != T) {
         dim3 b(32, 8, 1), g((nx + 31) / 32, (ny + 7) / 8, nz);
-        HT3D_LAUNCH(ctx, k_copy_inner_f32, g, b, 0, T, cur, nx, ny, nz);
+        HT3D_LAUNCH(ctx, k_copy_inner<float>, g, b, 0, T, cur, nx, ny, nz);
     }
 }
 
-// The mixed form's fused sweep (FP64 T, mixed stencils): x in place, y T -> S,
-// z S -> T, every axis one launch (both stages).
+// The mixed form's fused sweep (FP64 T, mixed stencils), every axis one launch
+// (both stages): x in place, y T -> S, z S -> T; where the rows are cut, x
+// T -> S, y S -> T, z T -> S and the result copied.
 template <int QUIRK>
 void all_mixed(ht3d_ctx* ctx, double* T, double* S, const double* const* V, double dt, const double* h,
                const WenoBC* bc, int nx, int ny, int nz) {
     using St = typename MixedStreamOf<QUIRK>::type;
     constexpr int warps = XWarps<double>::value;
-    const long long rows = (long long)ny * nz, per_block = 32LL * warps;
-    HT3D_LAUNCH(ctx, k_weno_xstream<St>, (unsigned)((rows + per_block - 1) / per_block), 32 * warps, 0, T, V[0], dt,
-                h[0], bc[0], nx, ny, nz);
-    HT3D_LAUNCH(ctx, (k_weno_march<1, St>), dim3((nx + 127) / 128, nz, march_chunks(ny)), 128, 0, T, S, V[1], dt,
-                h[1], bc[1], nx, ny, nz);
-    HT3D_LAUNCH(ctx, (k_weno_march<2, St>), dim3((nx + 127) / 128, ny, march_chunks(nz)), 128, 0, S, T, V[2], dt,
-                h[2], bc[2], nx, ny, nz);
+    const long long rows = (long long)ny * nz, per_block = 32LL * warps, wx = (nx + 31) / 32;
+    const int Kx = march_segments((rows + 31) / 32, nx, kWarpsMixed, 1),
+              Ky = march_segments(wx * nz, ny, kWarpsMixed, long_segments(ny)),
+              Kz = march_segments(wx * ny, nz, kWarpsMixed, long_segments(nz));
+    double* a = Kx == 1 ? T : S;  // after x
+    double* b = Kx == 1 ? S : T;  // after y; z goes back to a
+    const dim3 gx((unsigned)((rows + per_block - 1) / per_block), Kx);
+    if (Kx == 1) HT3D_LAUNCH(ctx, (k_weno_xstream<St, true>), gx, 32 * warps, 0, T, a, V[0], dt, h[0], bc[0], nx, ny, nz);
+    else HT3D_LAUNCH(ctx, (k_weno_xstream<St, false>), gx, 32 * warps, 0, T, a, V[0], dt, h[0], bc[0], nx, ny, nz);
+    HT3D_LAUNCH(ctx, (k_weno_march<1, St>), dim3((nx + 127) / 128, nz, Ky), 128, 0, a, b, V[1], dt, h[1], bc[1], nx, ny,
+                nz);
+    HT3D_LAUNCH(ctx, (k_weno_march<2, St>), dim3((nx + 127) / 128, ny, Kz), 128, 0, b, a, V[2], dt, h[2], bc[2], nx, ny,
+                nz);
+    if (a != T) {
+        dim3 bl(32, 8, 1), g((nx + 31) / 32, (ny + 7) / 8, nz);
+        HT3D_LAUNCH(ctx, k_copy_inner<double>, g, bl, 0, T, a, nx, ny, nz);
+    }
 }
 
 }  // namespace
