@@ -173,22 +173,57 @@ __global__ void k_reciprocal(double* __restrict__ iPC, const double* __restrict_
 struct F64Launch {
     int cells, threads, zchunk;  // cells per thread, threads per block, planes per block
     dim3 grid;
+    long long blocks() const { return (long long)grid.x * grid.z; }
 };
 inline F64Launch f64_shape(int cells, int threads, int zchunk, int nx, int ny, int nz) {
     const long long runs = (long long)((nx + cells - 1) / cells) * ny;
     return F64Launch{cells, threads, zchunk,
                      dim3((unsigned)((runs + threads - 1) / threads), 1, (unsigned)((nz + zchunk - 1) / zchunk))};
 }
-// Small grids: a cell per thread and a plane per block, as many warps as there
-// are (31 x 29 x 33: 4.9 us, 6.0 with two planes, 5.0 with two cells).  From 2^16
-// cells on two cells per thread, and chunks that leave each SM several blocks,
-// since one block's waits are hidden by another's arithmetic: two planes up to
-// 2^19 cells (63^3: 20.6 us, three 29), three up to 2^22 (95^3: 58.5, two 60.0;
-// 127 x 119 x 131: 131, two 138), eight above (255^3: 1009, three 1037).
-inline F64Launch f64_launch(int nx, int ny, int nz) {
+// Below 2^19 cells the shape whose busiest SM is done first.  One cell per thread
+// and a plane per block: an SM runs its share of the blocks together, 11.2 ns a
+// cell slot (40 x 38 x 36: 5.9 us, 7.3 with two planes; 48^3: 10.1, 12.2 with two
+// cells).  Two cells and two or three planes: two blocks at a time, 9.4 ns a slot,
+// 11.5 where an SM has one (63^3, two planes: 20.4, three 29.1, one cell 21.1;
+// 80 x 70 x 75, three: 31.0, two 38.8, one cell 32.6).  With more blocks than that
+// the rounds blend: three planes up to 2^22 cells (95^3: 58.2, two 59.7;
+// 127 x 119 x 131: 130, two 137), eight above (255^3: 1009, three 1037).
+inline F64Launch f64_launch(int sms, int nx, int ny, int nz) {
     const long long n = (long long)nx * ny * nz;
-    if (n < (1LL << 16)) return f64_shape(1, 128, 1, nx, ny, nz);
-    return f64_shape(2, 256, n < (1LL << 19) ? 2 : (n < (1LL << 22) ? 3 : 8), nx, ny, nz);
+    if (n >= (1LL << 19)) return f64_shape(2, 256, n < (1LL << 22) ? 3 : 8, nx, ny, nz);
+    F64Launch best = f64_shape(1, 128, 1, nx, ny, nz);
+    long long least = (best.blocks() + sms - 1) / sms * 128 * 112;
+    for (int c = 2; c <= 3; ++c) {
+        const F64Launch L = f64_shape(2, 256, c, nx, ny, nz);
+        const long long pairs = (L.blocks() + 2 * sms - 1) / (2 * sms);
+        const long long cost = L.blocks() <= sms ? 512 * c * 115 : pairs * 1024 * c * 94;
+        if (cost < least) least = cost, best = L;
+    }
+    return best;
+}
+
+// Dynamic shared memory that lets an SM hold no more of `blocks` blocks than its
+// share, for a launch_after whose blocks all run at once: the blocks of the next
+// launch, which start as soon as there is room, otherwise fill up some SMs and
+// leave others idle.  us per iteration without and with it, one cell per thread:
+// 48^3 12.7 -> 10.1; k_dim_iter at 48 x 48 x 24, heat and Darcy, 9.6 -> 7.0 and
+// 16.9 -> 11.4, at 40^3 9.8 -> 8.4 and 17.1 -> 14.3.
+template <typename... P>
+inline size_t even_smem(ht3d_ctx* ctx, void (*kern)(P...), int threads, long long blocks) {
+    int most = 1, per_sm = 0, reserved = 0, optin = 0;
+    cudaFuncAttributes fa;
+    HT3D_CUDA(cudaFuncGetAttributes(&fa, kern));
+    HT3D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&most, kern, threads, 0));
+    const int share = (int)std::max<long long>(1, (blocks + ctx->num_sms - 1) / ctx->num_sms);
+    if (share >= most || blocks > (long long)most * ctx->num_sms) return 0;
+    HT3D_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx->device));
+    HT3D_CUDA(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, ctx->device));
+    HT3D_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    const int fixed = (int)fa.sharedSizeBytes;
+    const int dyn = (std::min(per_sm / share - reserved, optin) - fixed) / 128 * 128;
+    if (dyn <= 0) return 0;
+    if (fixed + dyn > 48 * 1024) HT3D_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+    return (size_t)dyn;
 }
 
 template <int MODE>

@@ -15,7 +15,7 @@ int ht3d_dyrel_solve_fp64(ht3d_ctx* ctx, double* X, const double* R, const doubl
     double* X2 = (double*)ht3d_scratch(ctx, SLOT_X2, sizeof(double) * nex);
     IterLaunch L = iter_launch(ctx, nx, ny, nz);
     const bool fixed_variant = ctx->dyrel_variant != 0;  // the caller's thread layout
-    const F64Launch L64 = f64_launch(nx, ny, nz);
+    const F64Launch L64 = f64_launch(ctx->num_sms, nx, ny, nz);
     double* iPC = fixed_variant ? nullptr : (double*)ht3d_scratch(ctx, SLOT_G, sizeof(double) * n);
     const long long nsetup = (long long)((nx + 31) / 32) * ((ny + 7) / 8) * nz;
     // per-cell check terms (3n) followed by tree-pass work space
@@ -48,6 +48,15 @@ int ht3d_dyrel_solve_fp64(ht3d_ctx* ctx, double* X, const double* R, const doubl
     sc._dx = 1.0 / dx;
     sc._dy = 1.0 / dy;
     sc._dz = 1.0 / dz;
+    // the plain, storing and checking iterations
+    F64Kernel<0>::Fn kern64[3];
+    size_t smem64[3] = {0, 0, 0};
+    if (iPC) {
+        kern64[0] = F64Kernel<MODE_PLAIN>::get(cX != 0.0, true, L64);
+        kern64[1] = F64Kernel<MODE_STOREF>::get(cX != 0.0, true, L64);
+        kern64[2] = F64Kernel<MODE_CHECK>::get(cX != 0.0, true, L64);
+        for (int v = 0; v < 3; ++v) smem64[v] = even_smem(ctx, kern64[v], L64.threads, L64.blocks());
+    }
     double* cur = X;
     double* nxt = X2;
     DyrelCheck C;
@@ -61,11 +70,8 @@ int ht3d_dyrel_solve_fp64(ht3d_ctx* ctx, double* X, const double* R, const doubl
         sc.h2 = S.h2;
         sc.dtau = S.dtau;
         if (iPC) {
-            const bool cx = cX != 0.0;
-            const auto kern = chk ? F64Kernel<MODE_CHECK>::get(cx, true, L64)
-                                  : (storef ? F64Kernel<MODE_STOREF>::get(cx, true, L64)
-                                            : F64Kernel<MODE_PLAIN>::get(cx, true, L64));
-            launch_after(ctx, kern, L64.grid, L64.threads, 0, cur, nxt, R, kx, ky, kz, PC, iPC, F0, F,
+            const int v = chk ? 2 : (storef ? 1 : 0);
+            launch_after(ctx, kern64[v], L64.grid, L64.threads, smem64[v], cur, nxt, R, kx, ky, kz, PC, iPC, F0, F,
                          DyrelScalT<double>(sc), bc, nx, ny, nz, L64.zchunk, parts);
         } else if (chk)
             launch_iter<double, MODE_CHECK>(ctx, L, cur, nxt, R, kx, ky, kz, PC, F0, F, sc, bc, nx, ny, nz, parts);
@@ -142,13 +148,14 @@ extern "C" int ht3d_dyrel_iterate(ht3d_ctx* ctx, double* X_ex, const double* R, 
             iPC = (double*)ht3d_scratch(ctx, SLOT_G, sizeof(double) * n);
             HT3D_LAUNCH(ctx, k_reciprocal, (unsigned)std::min<long long>((n + 255) / 256, ctx->num_sms * 16LL), 256, 0, iPC, PC, n);
         }
-        const F64Launch L = f64_launch(nx, ny, nz);
+        const F64Launch L = f64_launch(ctx->num_sms, nx, ny, nz);
         const DyrelScalT<double> sc(DyrelScal{h1, h2, dtau, cX, 1.0 / dx, 1.0 / dy, 1.0 / dz});
         const auto kern = F64Kernel<MODE_PLAIN>::get(cX != 0.0, iPC != nullptr, L);
+        const size_t sm = even_smem(ctx, kern, L.threads, L.blocks());
         double* cur = X_ex;
         double* nxt = X2;
         for (int it = 0; it < n_iter; ++it) {
-            launch_after(ctx, kern, L.grid, L.threads, 0, cur, nxt, R, kx, ky, kz, PC, iPC, F0, (double*)nullptr, sc,
+            launch_after(ctx, kern, L.grid, L.threads, sm, cur, nxt, R, kx, ky, kz, PC, iPC, F0, (double*)nullptr, sc,
                          bc, nx, ny, nz, L.zchunk, (double*)nullptr);
             std::swap(cur, nxt);
         }

@@ -789,23 +789,14 @@ inline long long shell_blocks(int threads, int nx, int ny, int nz) {
     const long long n1 = nx + 2, n2 = ny + 2, n3 = nz + 2;
     return (2 * (n2 * n3 + n1 * n3 + n1 * n2) + threads - 1) / threads;
 }
-// A cell per thread below 2^20 cells (63^3, Darcy: 41.9 us, 45.7 with two), and
-// the chunk for which the SMs' last blocks end together: a block's time is about
-// its planes and a third of one (48 x 48 x 24, Darcy: one plane 16.8 us, two
-// 14.8; 56 x 56 x 28: 17.4 and 30.2).  Two cells above (127^3, heat: 152 us, 161
-// with one), in chunks of two planes or, with blocks to spare, eight.
-inline F64Launch dim_launch(int sms, int nx, int ny, int nz) {
+// A cell per thread and a plane per block below 2^20 cells (63^3, Darcy: 42.1 us,
+// 45.3 with two cells; 37 x 31 x 19: 9.0, 12.9 with two planes).  Two cells above
+// (127^3, heat: 151 us, 177 with one), in chunks of two planes or, with blocks to
+// spare, eight.
+inline F64Launch dim_launch(int nx, int ny, int nz) {
     const long long n = (long long)nx * ny * nz;
-    if (n >= (1LL << 20)) return f64_shape(2, 256, n < (1LL << 22) ? 2 : 8, nx, ny, nz);
-    F64Launch best = f64_shape(1, 128, 1, nx, ny, nz);
-    long long least = -1;
-    for (int c = 1; c <= 4; ++c) {
-        const F64Launch L = f64_shape(1, 128, c, nx, ny, nz);
-        const long long blocks = (long long)L.grid.x * L.grid.z + shell_blocks(128, nx, ny, nz);
-        const long long cost = (blocks + sms - 1) / sms * (3 * c + 1);
-        if (least < 0 || cost < least) least = cost, best = L;
-    }
-    return best;
+    if (n < (1LL << 20)) return f64_shape(1, 128, 1, nx, ny, nz);
+    return f64_shape(2, 256, n < (1LL << 22) ? 2 : 8, nx, ny, nz);
 }
 
 struct DimWork {
@@ -837,7 +828,7 @@ int dim_dyrel(ht3d_ctx* ctx, double* X, DimWork& W, const double* wN, DimScal s,
     const bool trans = s.tdt != 0.0;
     if (!PRESSURE) HT3D_LAUNCH(ctx, k_scale_rc, g1, 256, 0, W.tt, W.rC, s.transient, s._dt, n);
     else if (trans) HT3D_LAUNCH(ctx, k_rhof_terms, grid3z(nx, ny, nz), kBlock3, 0, W.tt, W.Tex, s.s_T, nx, ny, nz);
-    const F64Launch L = dim_launch(ctx->num_sms, nx, ny, nz);
+    const F64Launch L = dim_launch(nx, ny, nz);
     const int cb = (int)L.grid.x, wb = (int)(cb * L.grid.z);
     const unsigned grd = (unsigned)(wb + shell_blocks(L.threads, nx, ny, nz));
     typedef void (*Kern)(DimIterArgs, DimScal, DimBC, int, int, int, int, int, int);
@@ -854,6 +845,10 @@ int dim_dyrel(ht3d_ctx* ctx, double* X, DimWork& W, const double* wN, DimScal s,
     auto pick = [&](int mode) {
         return PRESSURE && trans ? kern_of(std::bool_constant<PRESSURE != 0>(), mode) : kern_of(std::false_type(), mode);
     };
+    // the plain, storing and checking iterations; the shell's blocks are short and come last
+    const Kern kern[3] = {pick(MODE_PLAIN), pick(MODE_STOREF), pick(MODE_CHECK)};
+    size_t smem[3];
+    for (int v = 0; v < 3; ++v) smem[v] = even_smem(ctx, kern[v], L.threads, wb);
     DimIterArgs A;
     A.ph = W.ph; A.wN = wN; A.kx = W.kx; A.ky = W.ky; A.kz = W.kz; A.PC = W.PC; A.iPC = W.iPC; A.F0 = W.F0; A.F = W.F;
     A.terms = W.terms; A.T0 = W.T0; A.rCt = W.tt; A.tt = W.tt; A.prf0 = W.prf0; A.rfy = W.rfy;
@@ -866,8 +861,8 @@ int dim_dyrel(ht3d_ctx* ctx, double* X, DimWork& W, const double* wN, DimScal s,
         const bool storef = !chk && (iter == prm->nitmax || is_check(iter + 1, prm->nitout));
         s.h1 = S.h1; s.h2 = S.h2; s.dtau = S.dtau;
         A.Xin = cur; A.Xout = nxt;
-        launch_after(ctx, pick(chk ? MODE_CHECK : (storef ? MODE_STOREF : MODE_PLAIN)), grd, L.threads, 0, A, s, b, nx,
-                     ny, nz, L.zchunk, wb, cb);
+        const int v = chk ? 2 : (storef ? 1 : 0);
+        launch_after(ctx, kern[v], grd, L.threads, smem[v], A, s, b, nx, ny, nz, L.zchunk, wb, cb);
         std::swap(cur, nxt);
         it_done = iter;
         if (chk) {

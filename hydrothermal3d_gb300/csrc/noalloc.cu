@@ -89,7 +89,10 @@ extern "C" int ht3d_dyrel_iterate_noalloc(double* X_ex, const double* R, const d
     if (s != HT3D_OK) return s;
     cudaStream_t st = (cudaStream_t)stream;
     const DyrelScalT<double> sc(DyrelScal{h1, h2, dtau, cX, 1.0 / dx, 1.0 / dy, 1.0 / dz});
-    const F64Launch L = f64_launch(nx, ny, nz);
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return HT3D_ERR_CUDA;
+    const F64Launch L = f64_launch(sms, nx, ny, nz);
     const auto kern = F64Kernel<MODE_PLAIN>::get(cX != 0.0, false, L);
     double* cur = X_ex;
     double* nxt = scratch;

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 import hydrothermal3d_gb300 as ht
-from hydrothermal3d_gb300 import api, abi
+from hydrothermal3d_gb300 import api, abi, v18
 
 pytestmark = pytest.mark.gpu
 
@@ -79,3 +79,50 @@ def test_fp64_iterate_with_and_without_reciprocals(ctx, n_iter):
     ctx.set_tuning(abi.TUNE_DYREL_VARIANT, 0)
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+# an SM's share of the blocks held down to 2, 3 and 4 by shared memory and not held
+# down; two cells per thread in chunks of two planes (odd nx) and of three
+@pytest.mark.parametrize("n", [(40, 31, 30), (48, 48, 24), (40, 38, 46), (48, 48, 48), (63, 63, 63), (79, 70, 74)])
+def test_fp64_iteration_at_the_shapes_of_its_rule(ctx, orc, n):
+    nx, ny, nz = n
+    rng = np.random.default_rng(17)
+    f = lambda *s: np.asfortranarray(rng.uniform(0.2, 1.7, s))
+    X, R = f(nx + 2, ny + 2, nz + 2), f(nx, ny, nz) - 1.0
+    k = [f(nx + 1, ny, nz), f(nx, ny + 1, nz), f(nx, ny, nz + 1)]
+    d, types, vals = (1.0 / nx, 0.9 / ny, 1.1 / nz), (0, 1, 1, 0, 0, 1), (0.3, -0.1, 1.0, 0.0, 0.5, 0.2)
+    prm = abi.DyrelParams.reference(nitout=4)
+    Xo, F, F0 = X.copy(order="F"), orc.zeros(*n), orc.zeros(*n)
+    s, sto = orc.dyrel_solve_dimless(Xo, R, *k, 25.0, *d, types, vals, prm, F, F0, n_iter_fixed=9)
+    Xd, Fd, F0d = ht.from_numpy(X), ht.zeros(*n), ht.zeros(*n)
+    std = api.dyrel_solve_dimless(ctx, Xd, ht.from_numpy(R), *[ht.from_numpy(a) for a in k], 25.0, *d, types, vals, prm,
+                                  Fd, F0d, abi.FP64, n_iter_fixed=9)
+    inner = (slice(1, -1),) * 3
+    np.testing.assert_array_equal(ht.to_numpy(Xd)[inner], Xo[inner])
+    np.testing.assert_array_equal(ht.to_numpy(Fd), F)
+    np.testing.assert_array_equal(ht.to_numpy(F0d), F0)
+    assert (std.nF_abs, std.lambda_min, std.lambda_max) == (sto.nF_abs, sto.lambda_min, sto.lambda_max)
+
+
+@pytest.mark.parametrize("n", [(40, 31, 30), (48, 48, 24), (40, 38, 46), (56, 56, 28), (63, 63, 31)])
+def test_dimensional_iteration_with_the_shared_blocks_held_down(ctx, orc, n):
+    """Twelve iterations of each system against the oracle's: the bounds of the
+    dimensional step (1e-12 of the largest value), at shares of 2 to 5 blocks
+    and with more blocks than run at once."""
+    nx, ny, nz = n
+    b = v18.box(*n, seed=3, nitout=6, nitmax=12)
+    V = [np.zeros(s, order="F") for s in ((nx + 1, ny, nz), (nx, ny + 1, nz), (nx, ny, nz + 1))]
+    T, P = b["T"].copy(order="F"), b["P"].copy(order="F")
+    Td, Pd = ht.from_numpy(T), ht.from_numpy(P)
+    Vd = [ht.zeros(*v.shape) for v in V]
+    a = [b[q] for q in ("phc", "phv", "wN", "kmul")]
+    p_o, p_d = b["params"], v18.box(*n, seed=3, nitout=6, nitmax=12)["params"]
+    p_o.it = p_d.it = 2
+    _, st_t, st_p = orc.step_v18(T, P, *a, *V, p_o)
+    gt, gp = api.step_v18(ctx, Td, Pd, *[ht.from_numpy(x) for x in a], *Vd, p_d)
+    assert (gt.iters, gp.iters) == (st_t.iters, st_p.iters)
+    inner = (slice(1, -1),) * 3
+    for d, o in ((ht.to_numpy(Td)[inner], T[inner]), (ht.to_numpy(Pd)[inner], P[inner])):
+        assert np.abs(d - o).max() <= 1e-12 * np.abs(o).max()
+    for d, o in zip(Vd, V):
+        assert np.abs(ht.to_numpy(d) - o).max() <= 1e-12 * np.abs(o).max()
