@@ -71,21 +71,7 @@ __device__ __forceinline__ double weno_ghost(double v, bool left, const WenoBC& 
 // (a, c, the three indicators, g) and one five-difference maximum e, and each
 // point evaluates only its weights: the indicators are computed once per
 // face instead of once per point and side.
-struct WenoStreamShared {
-    using value = float;      // storage and update type
-    using bc_type = WenoBCf;  // its end rules
-    using param = float;      // the grid factor h
-    float x[6];   // x_{i-3} .. x_{i+2}
-    float D[4];   // D_{i-2} .. D_{i+1}
-    float bl[3];  // bL_{i-2} .. bL_i
-    float bc[2];  // bC_{i-1}, bC_i
-    float br;     // bR_i
-    float g1[2];  // g_{i-1} / 3, g_i / 3
-    float g3;     // g_i / 2
-    float e;      // 1e-18 + 1e-6 max|D_{i-3} .. D_{i+1}|^2
-    float ap;     // a_i
-    float h;
-
+struct WenoWeights {
     __device__ __forceinline__ static float rcp(float v) {
         float r;
         asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
@@ -114,50 +100,156 @@ struct WenoStreamShared {
         const float m = fmaxf(fmaxf(fmaxf(fabsf(d0), fabsf(d1)), fmaxf(fabsf(d2), fabsf(d3))), fabsf(d4));
         return fmaf(1e-6f * m, m, 1e-18f);
     }
+};
 
-    __device__ __forceinline__ void init(const float (&x6)[6], float h_) {
-        h = h_;
+// FP32 form, both stages in one pair of lanes: the two stages of a line do the
+// same operations on different points, so the marching state holds stage 1 in
+// the low and stage 2 in the high half of 64-bit registers and a step is one
+// sequence of f32x2 instructions (each half rounds like the scalar operation;
+// the same text with float is the scalar step of a segment's first and last
+// points).  Only maxima, reciprocals and the velocities' signs go by halves.
+// The differences are unscaled; the grid factor h is in the floor and in dt h.
+// The weights d_k / (b_k + e)^2 are multiplied by the three squares: with
+// t_k = (b_k + e) / (4096 e) the ratio is
+//   N / W = (q1 n1 + q3 n3) / (q1 + 6 q2 + 3 q3), q1 = (t2 t3)^2 and so on,
+// and takes two reciprocals a point and side, one of them shared by the sides,
+// instead of four.  b_k <= 25 max|D|^2 and e >= 1e-6 max|D|^2, so
+// 2^-12 <= t_k < 7e3 and the products stay far inside the range.
+//
+// Bound by instructions, not by memory (511^3 moves 5.1 GB): 160 a cell and axis
+// and a 70 % busy issue before, about 125 now, two cycles each for the packed
+// ones.  Branches on the flow's direction cost more than the side that they
+// skip (2.08 ms with, 2.00 without).  Sweep, before and now: 127^3 87 -> 72 us,
+// 255^3 348 -> 296, 511^3 2.52 -> 2.11 ms.
+using W2 = unsigned long long;
+__device__ __forceinline__ W2 pk2(float lo, float hi) {
+    W2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpk2(W2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ float wadd(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float wsub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ float wmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float wfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ W2 wadd(W2 a, W2 b) { W2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ W2 wsub(W2 a, W2 b) { W2 r; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ W2 wmul(W2 a, W2 b) { W2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ W2 wfma(W2 a, W2 b, W2 c) {
+    W2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+template <class F> __device__ __forceinline__ F wset(float v);
+template <> __device__ __forceinline__ float wset<float>(float v) { return v; }
+template <> __device__ __forceinline__ W2 wset<W2>(float v) { return pk2(v, v); }
+__device__ __forceinline__ float wrcp(float v) { return WenoWeights::rcp(v); }
+__device__ __forceinline__ W2 wrcp(W2 v) {
+    float a, b;
+    unpk2(v, a, b);
+    return pk2(wrcp(a), wrcp(b));
+}
+__device__ __forceinline__ float wrcp_neg(float v) { return WenoWeights::rcp(-v); }
+__device__ __forceinline__ W2 wrcp_neg(W2 v) {
+    float a, b;
+    unpk2(v, a, b);
+    return pk2(wrcp_neg(a), wrcp_neg(b));
+}
+__device__ __forceinline__ float wmax5(float a, float b, float c, float d, float e) {
+    return fmaxf(fmaxf(fmaxf(fabsf(a), fabsf(b)), fmaxf(fabsf(c), fabsf(d))), fabsf(e));
+}
+__device__ __forceinline__ W2 wmax5(W2 a, W2 b, W2 c, W2 d, W2 e) {
+    float a0, a1, b0, b1, c0, c1, d0, d1, e0, e1;
+    unpk2(a, a0, a1);
+    unpk2(b, b0, b1);
+    unpk2(c, c0, c1);
+    unpk2(d, d0, d1);
+    unpk2(e, e0, e1);
+    return pk2(wmax5(a0, b0, c0, d0, e0), wmax5(a1, b1, c1, d1, e1));
+}
+// v d where v > 0 (v < 0), and 0 elsewhere whatever d is (NaN velocities included)
+__device__ __forceinline__ float wpos(float v, float d) { return v > 0.0f ? __fmul_rn(v, d) : 0.0f; }
+__device__ __forceinline__ float wneg(float v, float d) { return v < 0.0f ? __fmul_rn(v, d) : 0.0f; }
+__device__ __forceinline__ W2 wpos(W2 v, W2 d) {
+    float v0, v1, p0, p1;
+    unpk2(v, v0, v1);
+    unpk2(wmul(v, d), p0, p1);
+    return pk2(v0 > 0.0f ? p0 : 0.0f, v1 > 0.0f ? p1 : 0.0f);
+}
+__device__ __forceinline__ W2 wneg(W2 v, W2 d) {
+    float v0, v1, p0, p1;
+    unpk2(v, v0, v1);
+    unpk2(wmul(v, d), p0, p1);
+    return pk2(v0 < 0.0f ? p0 : 0.0f, v1 < 0.0f ? p1 : 0.0f);
+}
+
+template <class F>
+struct WenoLane {
+    F x[3];   // x_i .. x_{i+2}
+    F D[4];   // D_{i-2} .. D_{i+1}, unscaled
+    F bl[3];  // bL_{i-2} .. bL_i
+    F bc[2];  // bC_{i-1}, bC_i
+    F br;     // bR_i
+    F g[2];   // g_{i-1} / 3, g_i / 3
+    F re;     // 1 / (4096 e) of D_{i-3} .. D_{i+1}
+    F ap;     // a_i
+
+    __device__ __forceinline__ static void triple(F Dm, F D0, F Dp, F& a, F& L, F& C, F& R) {
+        a = wadd(wfma(wset<F>(-2.0f), D0, Dm), Dp);
+        const F c = wsub(Dm, Dp);
+        C = wfma(wmul(wset<F>(0.25f), c), c, wmul(wmul(wset<F>(13.0f / 12.0f), a), a));
+        L = wfma(a, wsub(a, c), C);
+        R = wfma(a, wadd(a, c), C);
+    }
+    // e0 = 4096e-18 / h^2
+    __device__ __forceinline__ static F floor5(F d0, F d1, F d2, F d3, F d4, F e0) {
+        const F m = wmax5(d0, d1, d2, d3, d4);
+        return wrcp(wfma(wmul(wset<F>(4096e-6f), m), m, e0));
+    }
+    // numerator and (positive) denominator of the weighted corrections
+    __device__ __forceinline__ static void ratio(F b1, F b2, F b3, F re, F n1, F n3, F& N, F& W) {
+        const F k = wset<F>(1.0f / 4096.0f);
+        const F t1 = wfma(b1, re, k), t2 = wfma(b2, re, k), t3 = wfma(b3, re, k);
+        const F r1 = wmul(t2, t3), r2 = wmul(t1, t3), r3 = wmul(t1, t2);
+        const F q1 = wmul(r1, r1), q2 = wmul(r2, r2), q3 = wmul(r3, r3);
+        W = wfma(wset<F>(3.0f), q3, wfma(wset<F>(6.0f), q2, q1));
+        N = wfma(q1, n1, wmul(q3, n3));
+    }
+    __device__ __forceinline__ void init(const F (&x6)[6], F e0) {
+        F d[5];
 #pragma unroll
-        for (int q = 0; q < 6; ++q) x[q] = x6[q];
-        float d[5];
-#pragma unroll
-        for (int q = 0; q < 5; ++q) d[q] = h * (x[q + 1] - x[q]);  // D_{i-3} .. D_{i+1}
-        float a2, a1, a0, unused0, unused1, unused2;
-        triple(d[0], d[1], d[2], a2, bl[0], unused0, unused1);   // centre i-2
-        triple(d[1], d[2], d[3], a1, bl[1], bc[0], unused2);     // centre i-1
-        triple(d[2], d[3], d[4], a0, bl[2], bc[1], br);          // centre i
-        g1[0] = (a1 - a2) * (1.0f / 3.0f);
-        g1[1] = (a0 - a1) * (1.0f / 3.0f);
-        g3 = 0.5f * (a0 - a1);
+        for (int q = 0; q < 5; ++q) d[q] = wsub(x6[q + 1], x6[q]);  // D_{i-3} .. D_{i+1}
+        F a2, a1, a0, u0, u1, u2;
+        triple(d[0], d[1], d[2], a2, bl[0], u0, u1);     // centre i-2
+        triple(d[1], d[2], d[3], a1, bl[1], bc[0], u2);  // centre i-1
+        triple(d[2], d[3], d[4], a0, bl[2], bc[1], br);  // centre i
+        g[0] = wmul(wsub(a1, a2), wset<F>(1.0f / 3.0f));
+        g[1] = wmul(wsub(a0, a1), wset<F>(1.0f / 3.0f));
         ap = a0;
-        e = floor5(d[0], d[1], d[2], d[3], d[4]);
+        re = floor5(d[0], d[1], d[2], d[3], d[4], e0);
 #pragma unroll
         for (int q = 0; q < 4; ++q) D[q] = d[q + 1];
-    }
-
-    __device__ __forceinline__ float back() const { return x[0]; }
-
-    __device__ __forceinline__ float step(float xn, float va, float vb, float dt) {
-        const float Dn = h * (xn - x[5]);  // D_{i+2}
-        float a1, bL1, bC1, bR1;
-        triple(D[2], D[3], Dn, a1, bL1, bC1, bR1);  // centre i+1
-        const float g = a1 - ap;
-        const float G1n = g * (1.0f / 3.0f), G3n = 0.5f * g;
-        const float e1 = floor5(D[0], D[1], D[2], D[3], Dn);
-        const float Vm = fminf(va, 0.0f), Vp = fmaxf(vb, 0.0f);
-        float dFm = 0.0f, dFp = 0.0f;
-        if (upwind_active(Vp)) {
-            const float p2 = fmaf(5.0f / 6.0f, D[1], fmaf(1.0f / 3.0f, D[2], (-1.0f / 6.0f) * D[0]));
-            dFm = mix(bl[0], bc[0], br, e, p2, -g1[0], -g3);
-        }
-        if (upwind_active(Vm)) {
-            const float p2 = fmaf(5.0f / 6.0f, D[2], fmaf(1.0f / 3.0f, D[1], (-1.0f / 6.0f) * D[3]));
-            dFp = mix(bR1, bc[1], bl[1], e1, p2, G1n, g3);
-        }
-        const float out = x[3] - dt * (Vp * dFm + Vm * dFp);
 #pragma unroll
-        for (int q = 0; q < 5; ++q) x[q] = x[q + 1];
-        x[5] = xn;
+        for (int q = 0; q < 3; ++q) x[q] = x6[q + 3];
+    }
+    // the stage value at i from x_{i+3} and the velocities of its faces; ndt = -dt h.
+    // Both sides are evaluated, without a branch on the flow's direction.
+    __device__ __forceinline__ F step(F xn, F va, F vb, F ndt, F e0) {
+        const F Dn = wsub(xn, x[2]);  // D_{i+2}
+        F a1, bL1, bC1, bR1;
+        triple(D[2], D[3], Dn, a1, bL1, bC1, bR1);  // centre i+1
+        const F gn = wmul(wsub(a1, ap), wset<F>(1.0f / 3.0f)), g3 = wmul(wset<F>(1.5f), g[1]);
+        const F re1 = floor5(D[0], D[1], D[2], D[3], Dn, e0);
+        F Nm, Wm, Np, Wp;
+        ratio(bl[0], bc[0], br, re, g[0], g3, Nm, Wm);  // the corrections are -g_{i-1} / 3 and -g_i / 2
+        ratio(bR1, bc[1], bl[1], re1, gn, g3, Np, Wp);
+        const F pm = wfma(wset<F>(5.0f / 6.0f), D[1], wfma(wset<F>(1.0f / 3.0f), D[2], wmul(wset<F>(-1.0f / 6.0f), D[0])));
+        const F pp = wfma(wset<F>(5.0f / 6.0f), D[2], wfma(wset<F>(1.0f / 3.0f), D[1], wmul(wset<F>(-1.0f / 6.0f), D[3])));
+        const F rhs = wadd(wpos(vb, wfma(Nm, wrcp_neg(Wm), pm)), wneg(va, wfma(Np, wrcp(Wp), pp)));
+        const F out = wfma(ndt, rhs, x[0]);
+        x[0] = x[1];
+        x[1] = x[2];
+        x[2] = xn;
 #pragma unroll
         for (int q = 0; q < 3; ++q) D[q] = D[q + 1];
         D[3] = Dn;
@@ -167,13 +259,17 @@ struct WenoStreamShared {
         bc[0] = bc[1];
         bc[1] = bC1;
         br = bR1;
-        g1[0] = g1[1];
-        g1[1] = G1n;
-        g3 = G3n;
-        e = e1;
+        g[0] = g[1];
+        g[1] = gn;
+        re = re1;
         ap = a1;
         return out;
     }
+};
+struct WenoStreamShared {  // March<WenoStreamShared> below
+    using value = float;
+    using bc_type = WenoBCf;
+    using param = float;
 };
 
 // Window form: the 7-point window and weno_point_f32, for the v2 stencil
@@ -238,9 +334,9 @@ struct WenoStreamMixed {
             d[q] = hf * (float)ee[q];
         }
         float a2, a1, a0, u0, u1, u2;
-        WenoStreamShared::triple(d[0], d[1], d[2], a2, bl[0], u0, u1);
-        WenoStreamShared::triple(d[1], d[2], d[3], a1, bl[1], bc[0], u2);
-        WenoStreamShared::triple(d[2], d[3], d[4], a0, bl[2], bc[1], br);
+        WenoWeights::triple(d[0], d[1], d[2], a2, bl[0], u0, u1);
+        WenoWeights::triple(d[1], d[2], d[3], a1, bl[1], bc[0], u2);
+        WenoWeights::triple(d[2], d[3], d[4], a0, bl[2], bc[1], br);
         const double A2 = __fma_rn(-2.0, ee[1], ee[0]) + ee[2];  // a_{i-2}
         const double A1 = __fma_rn(-2.0, ee[2], ee[1]) + ee[3];  // a_{i-1}
         const double A0 = __fma_rn(-2.0, ee[3], ee[2]) + ee[4];  // a_i
@@ -249,7 +345,7 @@ struct WenoStreamMixed {
         g1[1] = g0 * (1.0f / 3.0f);
         g3 = 0.5f * g0;
         ap = A0;
-        e = WenoStreamShared::floor5(d[0], d[1], d[2], d[3], d[4]);
+        e = WenoWeights::floor5(d[0], d[1], d[2], d[3], d[4]);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             E[q] = ee[q + 1];
@@ -263,20 +359,20 @@ struct WenoStreamMixed {
         const double en = xn - x[5];  // e_{i+2}
         const float Dn = hf * (float)en;
         float af, bL1, bC1, bR1;
-        WenoStreamShared::triple(D[2], D[3], Dn, af, bL1, bC1, bR1);  // centre i+1 (indicators)
+        WenoWeights::triple(D[2], D[3], Dn, af, bL1, bC1, bR1);  // centre i+1 (indicators)
         const double a1 = __fma_rn(-2.0, E[3], E[2]) + en;            // a_{i+1}
         const float gf = (float)(a1 - ap);                            // g_{i+1}
         const float G1n = gf * (1.0f / 3.0f), G3n = 0.5f * gf;
-        const float e1 = WenoStreamShared::floor5(D[0], D[1], D[2], D[3], Dn);
+        const float e1 = WenoWeights::floor5(D[0], D[1], D[2], D[3], Dn);
         const double Vm = neg_part(va), Vp = pos_part(vb);
         double rhs = 0.0;  // Vp dF- + Vm dF+ (unscaled derivatives)
         if (upwind_active(Vp)) {
             const double p2 = __fma_rn(2.0, E[2], __fma_rn(5.0, E[1], -E[0])) * (1.0 / 6.0);
-            rhs = Vp * (p2 + (double)WenoStreamShared::mix(bl[0], bc[0], br, e, 0.0f, -g1[0], -g3));
+            rhs = Vp * (p2 + (double)WenoWeights::mix(bl[0], bc[0], br, e, 0.0f, -g1[0], -g3));
         }
         if (upwind_active(Vm)) {
             const double p2 = __fma_rn(2.0, E[1], __fma_rn(5.0, E[2], -E[3])) * (1.0 / 6.0);
-            rhs = __fma_rn(Vm, p2 + (double)WenoStreamShared::mix(bR1, bc[1], bl[1], e1, 0.0f, G1n, g3), rhs);
+            rhs = __fma_rn(Vm, p2 + (double)WenoWeights::mix(bR1, bc[1], bl[1], e1, 0.0f, G1n, g3), rhs);
         }
         const double out = __fma_rn(-(dt * h), rhs, x[3]);  // dt h: loop invariant
 #pragma unroll
@@ -361,6 +457,8 @@ template <class Stream>
 struct March {
     using T = typename Stream::value;
     using BC = typename Stream::bc_type;
+    static constexpr int kAhead = 3;  // points that stage 1 is ahead of stage 2
+    __device__ __forceinline__ static int first_tail(int n) { return n - 3; }
     Stream s1, s2;
     T v0, v1, v2, v3;  // faces c .. c + 3 of the next step
     T gq0, gq1, gq2;   // tail: the T1 ghosts n, n + 1, n + 2
@@ -404,7 +502,7 @@ struct March {
         return (T)0.5 * t + (T)0.5 * t0c;
     }
     // at c = n - 3: s1 holds T0[n - 3 .. n + 2], s2 T1[n - 6 .. n - 1]
-    __device__ __forceinline__ void tail_enter(const BC& bc) {
+    __device__ __forceinline__ void tail_enter(const BC& bc, int) {
         tq0 = s1.x[0];
         tq1 = s1.x[1];
         tq2 = s1.x[2];
@@ -423,6 +521,128 @@ struct March {
         v1 = v2;
         v2 = v3;
         return out;
+    }
+};
+
+// The FP32 march: stage 1 at c + 4 and stage 2 at c in one paired step, which
+// takes T1[c + 3] from the step before.  The segment's first points of stage 1
+// and, past the last point of stage 1, the line's last four of stage 2 go alone.
+template <>
+struct March<WenoStreamShared> {
+    using BC = WenoBCf;
+    static constexpr int kAhead = 4;
+    __device__ __forceinline__ static int first_tail(int n) { return n < 4 ? 0 : n - 4; }
+    WenoLane<W2> s;   // stage 1 at c + 4, stage 2 at c
+    WenoLane<float> s2;  // stage 2 in the tail
+    float t1;            // T1[c + 3]
+    float t0[4];         // T0[c .. c + 3]
+    float v[5];          // faces c .. c + 4
+    float q[4];          // tail: T1 of the last point and the ghosts
+    float ndt, e0;
+
+    template <class Src>
+    __device__ __forceinline__ void start(const Src& src, int c0, const BC& bc, float dt, float h) {
+        ndt = -(dt * h);
+        e0 = fmaxf(4096e-18f / (h * h), 1e-36f);  // its reciprocal stays finite
+        const bool four = src.n >= 4;
+        WenoLane<float> a;
+        {
+            float x[6];
+#pragma unroll
+            for (int r = 0; r < 6; ++r) x[r] = src.t0(c0 - 6 + r);
+            a.init(x, e0);
+        }
+        float w[6];  // T1[c0 - 3 .. c0 + 2]
+#pragma unroll
+        for (int r = 0; r < 6; ++r)
+            w[r] = a.step(src.t0(c0 + r), src.v(c0 - 3 + r), src.v(c0 - 2 + r), ndt, e0);
+        if (c0 == 0) {
+            w[0] = weno_ghost(w[5], true, bc);
+            w[1] = weno_ghost(w[4], true, bc);
+            w[2] = weno_ghost(w[3], true, bc);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            t0[r] = src.t0(c0 + r);
+            v[r] = src.v(c0 + r);
+        }
+        v[4] = src.v(four ? c0 + 4 : c0);
+        t1 = four ? a.step(src.t0(c0 + 6), v[3], v[4], ndt, e0) : 0.0f;
+        WenoLane<float> b;
+        b.init(w, e0);
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            s.x[r] = pk2(a.x[r], b.x[r]);
+            s.bl[r] = pk2(a.bl[r], b.bl[r]);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) s.D[r] = pk2(a.D[r], b.D[r]);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            s.bc[r] = pk2(a.bc[r], b.bc[r]);
+            s.g[r] = pk2(a.g[r], b.g[r]);
+        }
+        s.br = pk2(a.br, b.br);
+        s.re = pk2(a.re, b.re);
+        s.ap = pk2(a.ap, b.ap);
+    }
+    // step c with its stage-1 point c + 4 inside the line (or past a segment's
+    // end, where nothing uses it): xa = T0[c + 7], va = face c + 5
+    __device__ __forceinline__ float step(float xa, float va, float) {
+        float t0n, unused, t1n, t;
+        unpk2(s.x[0], t0n, unused);  // T0[c + 4]
+        const W2 out = s.step(pk2(xa, t1), pk2(v[4], v[0]), pk2(va, v[1]), pk2(ndt, ndt), pk2(e0, e0));
+        unpk2(out, t1n, t);
+        const float r = __fmaf_rn(0.5f, t, __fmul_rn(0.5f, t0[0]));
+        t1 = t1n;
+#pragma unroll
+        for (int m = 0; m < 3; ++m) t0[m] = t0[m + 1];
+        t0[3] = t0n;
+#pragma unroll
+        for (int m = 0; m < 4; ++m) v[m] = v[m + 1];
+        v[4] = va;
+        return r;
+    }
+    __device__ __forceinline__ static float hi(W2 p) {
+        float a, b;
+        unpk2(p, a, b);
+        return b;
+    }
+    // at c = first_tail(n)
+    __device__ __forceinline__ void tail_enter(const BC& bc, int n) {
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            s2.x[r] = hi(s.x[r]);
+            s2.bl[r] = hi(s.bl[r]);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) s2.D[r] = hi(s.D[r]);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            s2.bc[r] = hi(s.bc[r]);
+            s2.g[r] = hi(s.g[r]);
+        }
+        s2.br = hi(s.br);
+        s2.re = hi(s.re);
+        s2.ap = hi(s.ap);
+        const float z0 = weno_ghost(s2.x[2], false, bc), z1 = weno_ghost(s2.x[1], false, bc);
+        const bool four = n >= 4;  // T1[n - 1] is still to come
+        q[0] = four ? t1 : z0;
+        q[1] = four ? weno_ghost(t1, false, bc) : z1;
+        q[2] = four ? z0 : weno_ghost(s2.x[0], false, bc);
+        q[3] = z1;
+    }
+    __device__ __forceinline__ float tail_step(float) {
+        const float t = s2.step(q[0], v[0], v[1], ndt, e0);
+        const float r = __fmaf_rn(0.5f, t, __fmul_rn(0.5f, t0[0]));
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            q[m] = q[m + 1];
+            t0[m] = t0[m + 1];
+        }
+#pragma unroll
+        for (int m = 0; m < 4; ++m) v[m] = v[m + 1];
+        return r;
     }
 };
 
@@ -447,27 +667,33 @@ struct LineSrc {
 };
 
 constexpr int kMarchUnroll = 4;  // steps per software-pipelined body of the y/z march
-constexpr int kMarchL = 64, kMarchMin = 8;
+constexpr int kMarchF32 = 128, kMarchMixed = 64, kMarchMin = 8;  // cells per segment, of long lines and at least
 constexpr long long kWarpsF32 = 1216, kWarpsMixed = 608;
-int long_segments(int n) { return n < 3 * kMarchL / 2 ? 1 : (n + kMarchL / 2) / kMarchL; }
+int long_segments(int n, int L) { return n < 3 * L / 2 ? 1 : (n + L / 2) / L; }
 // Segments that the lines of a sweep are cut into, `warps` warps of lines: K
 // where the lines alone fill the chip (whole rows along x, which the sweep may
-// update in place: 511^3 2.54 ms, 3.15 with rows cut at 64 cells; 64 cells per
-// thread along y and z); shorter ones, down to 8
-// (a segment's first steps read six cells before it), until there are `want`
-// warps.  A segment begins with about five steps' work that its neighbour does
-// as well, so more warps than that are slower: FP32 1216 (127^3: 87 us; 97 with
-// four times as many), mixed, where one warp per scheduler fills the FP64 pipe,
-// 608 (95^3: 276 us; 404 with twice as many).  Sweep before (segments of 48 and
-// more) and now, FP32 and mixed: 33 x 29 x 31 53 -> 39 and 169 -> 83 us, 63^3 81 ->
-// 39 and 313 -> 136, 95^3 109 -> 58 and 463 -> 276.
+// update in place: cut at 64 cells they took a fifth longer at 511^3; along y and
+// z 128 cells per thread in FP32, 1.92 ms, 2.00 with 64, and 64 in the mixed
+// form); shorter ones, down to 8 (a segment's first steps read six cells before
+// it), until there are `want` warps.  A segment begins with about five steps'
+// work that its neighbour does as well, so more warps than that are slower: FP32
+// 1216 (127^3: 74 us; 80 with twice as many), mixed, where one warp per scheduler
+// fills the FP64 pipe, 608 (95^3: 276 us; 404 with twice as many).  Sweep with
+// segments of 48 cells and more and with these, FP32 (before its paired form) and
+// mixed: 33 x 29 x 31 53 -> 39 and 169 -> 83 us, 63^3 81 -> 39 and 313 -> 136,
+// 95^3 109 -> 58 and 463 -> 276.
 int march_segments(long long warps, int n, long long want, int K) {
     while (warps * K < want && n / (K + 1) >= kMarchMin) ++K;
     return K;
 }
 
+// blocks per SM that the registers have to allow (0: the compiler's choice; 511^3
+// 1.92 ms, 1.93 with one more and spills, 1.97 with the compiler's choice)
+template <class Stream> struct MarchBlocks { static constexpr int line = 0, row = 0; };
+template <> struct MarchBlocks<WenoStreamShared> { static constexpr int line = 4, row = 3; };
+
 template <int AXIS, class Stream>
-__global__ void __launch_bounds__(128) k_weno_march(const typename Stream::value* __restrict__ src,
+__global__ void __launch_bounds__(128, MarchBlocks<Stream>::line) k_weno_march(const typename Stream::value* __restrict__ src,
                                                     typename Stream::value* __restrict__ dst,
                                                     const typename Stream::value* __restrict__ V,
                                                     typename Stream::value dt, typename Stream::param h,
@@ -491,9 +717,10 @@ __global__ void __launch_bounds__(128) k_weno_march(const typename Stream::value
     s.n = n;
     s.bc = bc;
     March<Stream> M;
+    constexpr int A = March<Stream>::kAhead, QT = A + 3, QV = A + 1;  // a step takes T0[c + QT] and face c + QV
     M.start(s, c0, bc, dt, h);
-    const int cA = c1 < n ? c1 : n - 3;  // steps whose stage-1 point c + 3 is inside the line
-    const int cB = min(cA, n - 6);       // ... and whose T0[c + 6] is too
+    const int cA = c1 < n ? c1 : M.first_tail(n);  // steps whose stage-1 point c + A is inside the line
+    const int cB = min(cA, n - QT);                // ... and whose T0[c + QT] is too
     int c = c0;
     if (cB - c0 >= 2 * kMarchUnroll) {
         // software pipeline: the T0 and face values of the next kMarchUnroll
@@ -501,15 +728,15 @@ __global__ void __launch_bounds__(128) k_weno_march(const typename Stream::value
         T qt[kMarchUnroll], qv[kMarchUnroll];
 #pragma unroll
         for (int u = 0; u < kMarchUnroll; ++u) {
-            qt[u] = s.ld(c + 6 + u);
-            qv[u] = s.v(c + 4 + u);
+            qt[u] = s.ld(c + QT + u);
+            qv[u] = s.v(c + QV + u);
         }
         for (; c + 2 * kMarchUnroll <= cB; c += kMarchUnroll) {
             T nt[kMarchUnroll], nv[kMarchUnroll];
 #pragma unroll
             for (int u = 0; u < kMarchUnroll; ++u) {
-                nt[u] = s.ld(c + kMarchUnroll + 6 + u);  // < cB + 6 <= n
-                nv[u] = s.v(c + kMarchUnroll + 4 + u);
+                nt[u] = s.ld(c + kMarchUnroll + QT + u);  // < cB + QT <= n
+                nv[u] = s.v(c + kMarchUnroll + QV + u);
             }
 #pragma unroll
             for (int u = 0; u < kMarchUnroll; ++u) s.put(c + u, M.step(qt[u], qv[u], dt));
@@ -523,12 +750,13 @@ __global__ void __launch_bounds__(128) k_weno_march(const typename Stream::value
         for (int u = 0; u < kMarchUnroll; ++u) s.put(c + u, M.step(qt[u], qv[u], dt));
         c += kMarchUnroll;
     }
-    for (; c < cB; ++c) s.put(c, M.step(s.ld(c + 6), s.v(c + 4), dt));
-    for (; c < cA; ++c) s.put(c, M.step(s.t0(c + 6), s.v(c + 4), dt));
+    for (; c < cB; ++c) s.put(c, M.step(s.ld(c + QT), s.v(c + QV), dt));
+    for (; c < cA; ++c) s.put(c, M.step(s.t0(c + QT), s.v(c + QV), dt));
     if (c1 == n) {
-        M.tail_enter(bc);
+        M.tail_enter(bc, n);
 #pragma unroll
-        for (int r = 0; r < 3; ++r) s.put(n - 3 + r, M.tail_step(dt));
+        for (int r = 0; r < A; ++r)
+            if (A == 3 || n >= A || r > 0) s.put(n - A + r, M.tail_step(dt));
     }
 }
 
@@ -583,7 +811,7 @@ struct RingSrc {
 // after tile v + 1 is stored), so whole rows are safe.
 // WHOLE: whole rows, in place (T is not read); else segments, T -> dst.
 template <class Stream, bool WHOLE>
-__global__ void __launch_bounds__(32 * XWarps<typename Stream::value>::value)
+__global__ void __launch_bounds__(32 * XWarps<typename Stream::value>::value, MarchBlocks<Stream>::row)
     k_weno_xstream(const typename Stream::value* __restrict__ T, typename Stream::value* __restrict__ dst,
                    const typename Stream::value* __restrict__ Vx,
                    typename Stream::value dt, typename Stream::param h, typename Stream::bc_type bc, int nx, int ny,
@@ -620,8 +848,9 @@ __global__ void __launch_bounds__(32 * XWarps<typename Stream::value>::value)
     }
     const E* Tw = (WHOLE ? dst : T) + t0off;
     const E* Vw = Vx + (long long)(nx + 1) * row0;
-    const int tq_lo = max(0, c0 - 6), tq_hi = min(n, c1 + 6);  // T0 positions a segment reads
-    const int vq_lo = max(0, c0 - 3), vq_hi = min(n, c1 + 3);  // faces (inclusive)
+    constexpr int A = March<Stream>::kAhead, QT = A + 3, QV = A + 1;  // a step takes T0[c + QT] and face c + QV
+    const int tq_lo = max(0, c0 - 6), tq_hi = min(n, c1 + QT);  // T0 positions a segment reads
+    const int vq_lo = max(0, c0 - 3), vq_hi = min(n, c1 + A);   // faces (inclusive)
     auto load_tile = [&](int u) {
         const int q = b0 + kXW * u + cc;
         E* td = tr + (u % 3) * kXW + cc;
@@ -661,17 +890,17 @@ __global__ void __launch_bounds__(32 * XWarps<typename Stream::value>::value)
     M.start(src, c0, bc, dt, h);
     __syncwarp();
     load_tile(3);
-    const int cA = c1 < n ? c1 : n - 3;
+    const int cA = c1 < n ? c1 : M.first_tail(n);
     for (int v = 0, cb = c0; cb < c1; ++v, cb += kXW) {
         E* tcur = src.t + ((v + 1) % 3) * kXW;  // positions cb .. cb + 7
         const E* tnxt = src.t + ((v + 2) % 3) * kXW;
         const E* vcur = src.vp + ((v + 1) % 3) * kXW;
         const E* vnxt = src.vp + ((v + 2) % 3) * kXW;
-        if (cb + kXW <= cA && cb + kXW + 6 <= n) {  // eight steps without ghosts
+        if (cb + kXW <= cA && cb + kXW + QT - 1 < n) {  // eight steps without ghosts
 #pragma unroll
             for (int m = 0; m < kXW; ++m) {
-                const E xa = m + 6 < kXW ? tcur[m + 6] : tnxt[m + 6 - kXW];
-                const E va = m + 4 < kXW ? vcur[m + 4] : vnxt[m + 4 - kXW];
+                const E xa = m + QT < kXW ? tcur[m + QT] : tnxt[m + QT - kXW];
+                const E va = m + QV < kXW ? vcur[m + QV] : vnxt[m + QV - kXW];
                 tcur[m] = M.step(xa, va, dt);
             }
         } else {
@@ -679,9 +908,9 @@ __global__ void __launch_bounds__(32 * XWarps<typename Stream::value>::value)
                 const int c = cb + m;
                 E out;
                 if (c < cA) {
-                    out = M.step(src.t0(c + 6), src.v(c + 4), dt);
+                    out = M.step(src.t0(c + QT), src.v(c + QV), dt);
                 } else {
-                    if (c == n - 3) M.tail_enter(bc);
+                    if (c == M.first_tail(n)) M.tail_enter(bc, n);
                     out = M.tail_step(dt);
                 }
                 src.put(c, out);
@@ -817,7 +1046,7 @@ float* axis_f32(ht3d_ctx* ctx, float* cur, float* other, float* tmp, const float
         if (!periodic) {
             const int n = AXIS == 1 ? ny : nz;
             const dim3 g((nx + 127) / 128, AXIS == 1 ? nz : ny,
-                         march_segments((nx + 31) / 32 * (AXIS == 1 ? nz : ny), n, kWarpsF32, long_segments(n)));
+                         march_segments((nx + 31) / 32 * (AXIS == 1 ? nz : ny), n, kWarpsF32, long_segments(n, kMarchF32)));
             HT3D_LAUNCH(ctx, (k_weno_march<AXIS, typename StreamOf<QUIRK>::type>), g, 128, 0, cur, other, V, dt, h,
                         bcf(bc), nx, ny, nz);
             return other;
@@ -853,8 +1082,8 @@ void all_mixed(ht3d_ctx* ctx, double* T, double* S, const double* const* V, doub
     constexpr int warps = XWarps<double>::value;
     const long long rows = (long long)ny * nz, per_block = 32LL * warps, wx = (nx + 31) / 32;
     const int Kx = march_segments((rows + 31) / 32, nx, kWarpsMixed, 1),
-              Ky = march_segments(wx * nz, ny, kWarpsMixed, long_segments(ny)),
-              Kz = march_segments(wx * ny, nz, kWarpsMixed, long_segments(nz));
+              Ky = march_segments(wx * nz, ny, kWarpsMixed, long_segments(ny, kMarchMixed)),
+              Kz = march_segments(wx * ny, nz, kWarpsMixed, long_segments(nz, kMarchMixed));
     double* a = Kx == 1 ? T : S;  // after x
     double* b = Kx == 1 ? S : T;  // after y; z goes back to a
     const dim3 gx((unsigned)((rows + per_block - 1) / per_block), Kx);
