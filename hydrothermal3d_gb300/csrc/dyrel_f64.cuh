@@ -202,30 +202,6 @@ inline F64Launch f64_launch(int sms, int nx, int ny, int nz) {
     return best;
 }
 
-// Dynamic shared memory that lets an SM hold no more of `blocks` blocks than its
-// share, for a launch_after whose blocks all run at once: the blocks of the next
-// launch, which start as soon as there is room, otherwise fill up some SMs and
-// leave others idle.  us per iteration without and with it, one cell per thread:
-// 48^3 12.7 -> 10.1; k_dim_iter at 48 x 48 x 24, heat and Darcy, 9.6 -> 7.0 and
-// 16.9 -> 11.4, at 40^3 9.8 -> 8.4 and 17.1 -> 14.3.
-template <typename... P>
-inline size_t even_smem(ht3d_ctx* ctx, void (*kern)(P...), int threads, long long blocks) {
-    int most = 1, per_sm = 0, reserved = 0, optin = 0;
-    cudaFuncAttributes fa;
-    HT3D_CUDA(cudaFuncGetAttributes(&fa, kern));
-    HT3D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&most, kern, threads, 0));
-    const int share = (int)std::max<long long>(1, (blocks + ctx->num_sms - 1) / ctx->num_sms);
-    if (share >= most || blocks > (long long)most * ctx->num_sms) return 0;
-    HT3D_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx->device));
-    HT3D_CUDA(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, ctx->device));
-    HT3D_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
-    const int fixed = (int)fa.sharedSizeBytes;
-    const int dyn = (std::min(per_sm / share - reserved, optin) - fixed) / 128 * 128;
-    if (dyn <= 0) return 0;
-    if (fixed + dyn > 48 * 1024) HT3D_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
-    return (size_t)dyn;
-}
-
 template <int MODE>
 struct F64Kernel {
     typedef void (*Fn)(const double*, double*, const double*, const double*, const double*, const double*, const double*,

@@ -20,14 +20,20 @@ namespace {
 //           corrections; FP32 smoothness indicators and weights (weno5_mixed)
 //   STAGE 1: dst = src - dt*(Vp*dFm + Vm*dFp)
 //   STAGE 2: dst = 0.5*(src - dt*(...)) + 0.5*T0   (TimeAveraging!, order 2)
-template <int AXIS, int QUIRK, int STAGE, int PREC>
-__global__ void __launch_bounds__(256) k_weno_stage(const double* __restrict__ src, double* dst, const double* T0,
-                                                    const double* __restrict__ V, double dt, double h, WenoBC bc,
-                                                    int nx, int ny, int nz) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = blockIdx.z;
-    if (i >= nx || j >= ny || k >= nz) return;
+// A block has a run of T cells of a plane, row after row without gaps: bound by
+// the FP64 pipe, where an idle lane costs as much as a busy one.  Launched by
+// launch_after, six to a sweep.  Blocks of 32 x 8 cells, plain launches and
+// second derivatives by the whole warp before, in a rough flow: 48 x 48 x 24 180 us
+// of kernels, now 126 with the gaps between them; 127^3, smooth, 3.40 -> 3.07 ms.
+template <int AXIS, int QUIRK, int STAGE, int PREC, int T>
+__global__ void __launch_bounds__(T) k_weno_stage(const double* __restrict__ src, double* dst, const double* T0,
+                                                  const double* __restrict__ V, double dt, double h, WenoBC bc, int nx,
+                                                  int ny, int nz) {
+    after_previous();
+    const int tid = threadIdx.x, k = blockIdx.y;
+    const int c = blockIdx.x * T + tid, j0 = c / nx;
+    const bool live = j0 < ny;
+    const int j = live ? j0 : ny - 1, i = live ? c - j0 * nx : nx - 1;  // threads past the plane store nothing
     const int n1 = nx + 2, n2 = ny + 2;
     const long long e = (i + 1) + (long long)n1 * ((j + 1) + (long long)n2 * (k + 1));
     const int idx = AXIS == 0 ? i : (AXIS == 1 ? j : k);
@@ -50,17 +56,45 @@ __global__ void __launch_bounds__(256) k_weno_stage(const double* __restrict__ s
         // x[o] holds X[I+o-3].  A point has one inflow side almost always: its
         // lane selects that side's differences, so a warp whose flow changes sign
         // evaluates one derivative per lane and not both for all (127^3 sweep:
-        // 4.38 -> 3.40 ms).
+        // 4.38 -> 3.40 ms).  The second derivatives of the points with two inflow
+        // sides (in a rough flow some in every warp) are evaluated together, by
+        // as many warps of the block as they fill.
+        __shared__ double queue[5][T];
+        __shared__ int queued;
+        if (tid == 0) queued = 0;
         double d[6];
 #pragma unroll
         for (int o = 0; o < 6; ++o) d[o] = h * (x[o + 1] - x[o]);
         const double m5 = QUIRK ? h * (x[5] - x[2]) : d[4];
-        const bool minus = upwind_active(Vp), plus = upwind_active(Vm);
+        const bool minus = live && upwind_active(Vp), plus = live && upwind_active(Vm), both = minus && plus;
+        const bool any = __syncthreads_or(both);
+        int slot = 0;
+        if (any) {
+            const unsigned m = __ballot_sync(0xffffffffu, both);
+            const int lane = tid & 31;
+            int base = 0;
+            if (lane == 0 && m) base = atomicAdd(&queued, __popc(m));
+            slot = __shfl_sync(0xffffffffu, base, 0) + __popc(m & ((1u << lane) - 1u));
+            if (both) {
+                queue[0][slot] = d[5];
+                queue[1][slot] = d[4];
+                queue[2][slot] = d[3];
+                queue[3][slot] = d[2];
+                queue[4][slot] = d[1];
+            }
+            __syncthreads();
+        }
         rhs = 0.0;  // Vp dF- + Vm dF+, a product with a zero factor left out
         if (minus || plus)
             rhs = (minus ? Vp : Vm) * weno5_ref(minus ? d[0] : d[5], minus ? d[1] : d[4], minus ? d[2] : d[3],
                                                 minus ? d[3] : d[2], minus ? m5 : d[1]);
-        if (minus && plus) rhs += Vm * weno5_ref(d[5], d[4], d[3], d[2], d[1]);
+        if (any) {
+            // the warps that take the queue differ from block to block, and with them their schedulers
+            const int q = (int)((tid + 32u * (blockIdx.x + blockIdx.y)) % T);
+            if (q < queued) queue[0][q] = weno5_ref(queue[0][q], queue[1][q], queue[2][q], queue[3][q], queue[4][q]);
+            __syncthreads();
+            if (both) rhs += Vm * queue[0][slot];
+        }
     } else {
         // FP64 differences e[o] = X[I+o-2] - X[I+o-3]; FP32 copies scaled by h
         // for the smoothness indicators (weno5_mixed)
@@ -80,6 +114,7 @@ __global__ void __launch_bounds__(256) k_weno_stage(const double* __restrict__ s
                                              : 0.0;
         rhs = Vp * dFm + Vm * dFp;
     }
+    if (!live) return;
     const double t = x[3] - dt * rhs;
     if (STAGE == 1) dst[e] = t;
     else dst[e] = PREC == 0 ? __fma_rn(0.5, t, 0.5 * T0[e]) : 0.5 * t + 0.5 * T0[e];  // 0.5 t is exact
@@ -218,12 +253,24 @@ inline dim3 g1(ht3d_ctx* ctx, long long n) {
 }
 
 template <int AXIS, int QUIRK, int PREC>
-void weno_axis(ht3d_ctx* ctx, double* T, double* T1, const double* V, double dt, double h, WenoBC bc, int nx, int ny,
+void weno_axis(ht3d_ctx* ctx, double* T0, double* T1, const double* V, double dt, double h, WenoBC bc, int nx, int ny,
                int nz) {
-    dim3 b(32, 8, 1), g((nx + 31) / 32, (ny + 7) / 8, nz);
-    HT3D_LAUNCH(ctx, (k_weno_stage<AXIS, QUIRK, 1, PREC>), g, b, 0, T, T1, (const double*)nullptr, V, dt, h, bc, nx,
-                ny, nz);
-    HT3D_LAUNCH(ctx, (k_weno_stage<AXIS, QUIRK, 2, PREC>), g, b, 0, T1, T, T, V, dt, h, bc, nx, ny, nz);
+    // Short blocks spread a small grid evenly over the SMs (sweep at 48 x 48 x 24: 113
+    // us, 139 with 256 threads), long ones fill the queue's warps better (127^3, rough
+    // flow: 3.58 ms, 3.69 with 128).
+    auto go = [&](auto threads) {
+        constexpr int T = decltype(threads)::value;
+        const dim3 g((unsigned)(((long long)nx * ny + T - 1) / T), nz);
+        const long long blocks = (long long)g.x * g.y;
+        launch_after(ctx, k_weno_stage<AXIS, QUIRK, 1, PREC, T>, g, T,
+                     even_smem(ctx, k_weno_stage<AXIS, QUIRK, 1, PREC, T>, T, blocks), T0, T1, (const double*)nullptr, V,
+                     dt, h, bc, nx, ny, nz);
+        launch_after(ctx, k_weno_stage<AXIS, QUIRK, 2, PREC, T>, g, T,
+                     even_smem(ctx, k_weno_stage<AXIS, QUIRK, 2, PREC, T>, T, blocks), T1, T0, T0, V, dt, h, bc, nx, ny,
+                     nz);
+    };
+    if ((long long)nx * ny * nz < (1LL << 17)) go(std::integral_constant<int, 128>());
+    else go(std::integral_constant<int, 256>());
 }
 
 template <int QUIRK, int PREC>

@@ -126,3 +126,30 @@ def test_dimensional_iteration_with_the_shared_blocks_held_down(ctx, orc, n):
         assert np.abs(d - o).max() <= 1e-12 * np.abs(o).max()
     for d, o in zip(Vd, V):
         assert np.abs(ht.to_numpy(d) - o).max() <= 1e-12 * np.abs(o).max()
+
+
+# runs of 128 and of 256 cells that end inside a row and a plane; the smallest grid;
+# one inflow side everywhere, two at some points of each warp, two at every point
+@pytest.mark.parametrize("n", [(3, 3, 3), (5, 43, 4), (33, 17, 9), (129, 3, 5), (48, 48, 24), (67, 61, 33)])
+@pytest.mark.parametrize("flow", ["one", "rough", "spread"])
+@pytest.mark.parametrize("variant", [abi.WENO_V1, abi.WENO_V2_REF])
+def test_fused_sweep_with_two_inflow_sides(ctx, orc, n, flow, variant):
+    nx, ny, nz = n
+    rng = np.random.default_rng(29)
+    T = np.asfortranarray(rng.uniform(0, 1, (nx + 2, ny + 2, nz + 2)))
+    V = [rng.uniform(-1, 1, [m + (a == b) for b, m in enumerate(n)]) for a in range(3)]
+    if flow == "one":
+        V = [abs(v) for v in V]
+    elif flow == "spread":  # every other face flows backwards: a cell has two inflow sides or none
+        V = [abs(v) * (1 - 2 * (np.indices(v.shape)[a] % 2 == 0)) for a, v in enumerate(V)]
+    V = [np.asfortranarray(v) for v in V]
+    h, dt, types, vals = [float(m) for m in n], 0.2 / max(n), [0, 0, 1, 1, 2, 2], [0, 0, 1.0, 0.3, 0, 0]
+    To = T.copy(order="F")
+    if variant == abi.WENO_V1:
+        orc.call("AdvectWithWeno5_v1", To, *V, dt, *h, orc.int6(*types), orc.dbl6(*vals), *n)
+    else:
+        orc.call("AdvectWithWeno5_v2", To, *V, dt, *h, orc.int6(*types), orc.dbl6(*vals), 1, *n)
+    Td = ht.from_numpy(T)
+    api.weno5_advect(ctx, Td, *[ht.from_numpy(v) for v in V], dt, *h, types, vals, variant, abi.FP64)
+    inner = (slice(1, -1),) * 3
+    np.testing.assert_array_equal(ht.to_numpy(Td)[inner], To[inner])
