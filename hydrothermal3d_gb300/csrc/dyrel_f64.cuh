@@ -180,24 +180,30 @@ inline F64Launch f64_shape(int cells, int threads, int zchunk, int nx, int ny, i
     return F64Launch{cells, threads, zchunk,
                      dim3((unsigned)((runs + threads - 1) / threads), 1, (unsigned)((nz + zchunk - 1) / zchunk))};
 }
-// Below 2^19 cells the shape whose busiest SM is done first.  One cell per thread
-// and a plane per block: an SM runs its share of the blocks together, 11.2 ns a
-// cell slot (40 x 38 x 36: 5.9 us, 7.3 with two planes; 48^3: 10.1, 12.2 with two
-// cells).  Two cells and two or three planes: two blocks at a time, 9.4 ns a slot,
-// 11.5 where an SM has one (63^3, two planes: 20.4, three 29.1, one cell 21.1;
-// 80 x 70 x 75, three: 31.0, two 38.8, one cell 32.6).  With more blocks than that
-// the rounds blend: three planes up to 2^22 cells (95^3: 58.2, two 59.7;
-// 127 x 119 x 131: 130, two 137), eight above (255^3: 1009, three 1037).
+// Below 2^19 cells the shape whose busiest SM is done first: an SM's share of the
+// cell slots, times what a slot takes where the SM's blocks run together, and 1.2 us
+// a plane of a block.  One cell per thread in blocks of 128 for the smallest grids
+// (31 x 29 x 33: 4.6 us) and of 256 (72 x 70 x 75: 28.6, 29.9 with 128); two cells
+// in blocks of 64 and two planes while an SM holds its share of them at once (56^3:
+// 14.7, 15.3 with one cell; 63^3: 18.8, 20.4), and in blocks of 256 and two or three
+// planes while an SM holds its two at once (80 x 70 x 75: 31.0, 32.6 with one cell;
+// but 80^3, a second round of them: 42.1, 39.0).  From 2^19 cells on the rounds blend:
+// three planes up to 2^22 (95^3: 58.2, 63.0 with one cell; 127 x 119 x 131: 130, two
+// planes 137), eight above (255^3: 1009, three 1037).
 inline F64Launch f64_launch(int sms, int nx, int ny, int nz) {
     const long long n = (long long)nx * ny * nz;
     if (n >= (1LL << 19)) return f64_shape(2, 256, n < (1LL << 22) ? 3 : 8, nx, ny, nz);
-    F64Launch best = f64_shape(1, 128, 1, nx, ny, nz);
-    long long least = (best.blocks() + sms - 1) / sms * 128 * 112;
-    for (int c = 2; c <= 3; ++c) {
-        const F64Launch L = f64_shape(2, 256, c, nx, ny, nz);
-        const long long pairs = (L.blocks() + 2 * sms - 1) / (2 * sms);
-        const long long cost = L.blocks() <= sms ? 512 * c * 115 : pairs * 1024 * c * 94;
-        if (cost < least) least = cost, best = L;
+    struct Shape { int cells, threads, planes, most, ps; };  // most: blocks that an SM may have; ps a slot
+    const Shape shapes[] = {{1, 128, 1, 1 << 30, 11200}, {1, 256, 1, 1 << 30, 10800}, {2, 64, 2, 9, 9500},
+                            {2, 256, 2, 2, 8800}, {2, 256, 3, 2, 8800}};
+    F64Launch best{};
+    long long least = -1;
+    for (const Shape& h : shapes) {
+        const F64Launch L = f64_shape(h.cells, h.threads, h.planes, nx, ny, nz);
+        const long long share = (L.blocks() + sms - 1) / sms;
+        if (share > h.most) continue;
+        const long long cost = share * h.cells * h.threads * h.planes * h.ps + 1200000LL * h.planes;
+        if (least < 0 || cost < least) least = cost, best = L;
     }
     return best;
 }
@@ -208,7 +214,9 @@ struct F64Kernel {
                        const double*, double*, double*, DyrelScalT<double>, BC6<double>, int, int, int, int, double*);
     template <bool CX, bool INV>
     static Fn by_shape(const F64Launch& L) {
-        return L.cells == 1 ? (Fn)k_dyrel_f64<MODE, CX, INV, 128, 1> : (Fn)k_dyrel_f64<MODE, CX, INV, 256, 2>;
+        if (L.cells == 1)
+            return L.threads == 128 ? (Fn)k_dyrel_f64<MODE, CX, INV, 128, 1> : (Fn)k_dyrel_f64<MODE, CX, INV, 256, 1>;
+        return L.threads == 64 ? (Fn)k_dyrel_f64<MODE, CX, INV, 64, 2> : (Fn)k_dyrel_f64<MODE, CX, INV, 256, 2>;
     }
     static Fn get(bool cx, bool inv, const F64Launch& L) {
         return cx ? (inv ? by_shape<true, true>(L) : by_shape<true, false>(L))

@@ -81,9 +81,10 @@ def test_fp64_iterate_with_and_without_reciprocals(ctx, n_iter):
         np.testing.assert_array_equal(a, b)
 
 
-# an SM's share of the blocks held down to 2, 3 and 4 by shared memory and not held
-# down; two cells per thread in chunks of two planes (odd nx) and of three
-@pytest.mark.parametrize("n", [(40, 31, 30), (48, 48, 24), (40, 38, 46), (48, 48, 48), (63, 63, 63), (79, 70, 74)])
+# an SM's share of the blocks held down by shared memory and not; one cell per thread
+# in blocks of 128 and 256, two (odd nx) in blocks of 64 and of 256, at every size class
+@pytest.mark.parametrize("n", [(40, 31, 30), (48, 48, 24), (40, 38, 46), (48, 48, 48), (63, 63, 63), (79, 70, 74),
+                               (80, 80, 80)])
 def test_fp64_iteration_at_the_shapes_of_its_rule(ctx, orc, n):
     nx, ny, nz = n
     rng = np.random.default_rng(17)
