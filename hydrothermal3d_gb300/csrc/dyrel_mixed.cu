@@ -323,13 +323,16 @@ __device__ __forceinline__ void mixed_quad_march(const float* __restrict__ Din, 
 #define HT3D_MIX_MINB 16
 #endif
 // One instance: thread t of plane k = blockIdx.y handles quad t of the plane.
-template <bool STOREF>
+// AFTER: for launch_after.  It hides the start of a launch and costs a few registers
+// too many: us per iteration plain and after, 63^3 3.9 and 2.6, 127^3 9.5 and 8.3,
+// 150 x 149 x 151 14.8 and 16.0, 266 x 174 x 216 48.0 and 50.7.
+template <bool STOREF, bool AFTER>
 __global__ void __launch_bounds__(HT3D_MIX_BS, HT3D_MIX_MINB) k_mixed_inner(const float* __restrict__ Din, float* __restrict__ Dio,
                                                         const float* __restrict__ Rin, const float* __restrict__ kx,
                                                         const float* __restrict__ ky, const float* __restrict__ kz,
                                                         float* __restrict__ F, MixScal s, int prev0, BC6<float> bc,
                                                         Pad p) {
-    after_previous();
+    if (AFTER) after_previous();
     mixed_quad<STOREF>(Din, Dio, Rin, kx, ky, kz, F, s, prev0 != 0, bc, p, blockIdx.x * blockDim.x + threadIdx.x,
                        blockIdx.y, threadIdx.x & 31);
 }
@@ -1187,6 +1190,8 @@ int ht3d_dyrel_solve_mixed(ht3d_ctx* ctx, double* X, const double* R, const doub
     sc._dy = 1.0 / dy;
     sc._dz = 1.0 / dz;
     const dim3 ib(HT3D_MIX_BS), ig((unsigned)(((long long)P.nq * ny + HT3D_MIX_BS - 1) / HT3D_MIX_BS), (unsigned)nz);
+    // up to three and a half waves of k_mixed_inner (127^3 8.3 us after, 9.5 plain; 133^3 10.6 and 9.9)
+    const bool single_after = (long long)ig.x * ig.y <= 56LL * ctx->num_sms;
     // two iterations per pass (k_mixed_inner2) inside runs of inner iterations
     bool pairs = want_pairs;
     int zc = ctx->mixed_temporal >= 2 ? ctx->mixed_temporal : 0;
@@ -1326,12 +1331,16 @@ int ht3d_dyrel_solve_mixed(ht3d_ctx* ctx, double* X, const double* R, const doub
                 timer.count(2);
                 ++iter;  // the pass did iterations iter and iter + 1
             } else {
-                if (storef)
-                    launch_after(ctx, k_mixed_inner<true>, ig, ib, 0, Dbuf[cur], Dbuf[prv], Rin, kx32, ky32, kz32, Fs,
-                                s32, prev0 ? 1 : 0, bch, P);
-                else
-                    launch_after(ctx, k_mixed_inner<false>, ig, ib, 0, Dbuf[cur], Dbuf[prv], Rin, kx32, ky32, kz32, Fs,
-                                s32, prev0 ? 1 : 0, bch, P);
+                auto go = [&](auto kern, auto kern_after) {
+                    if (single_after)
+                        launch_after(ctx, kern_after, ig, ib, 0, Dbuf[cur], Dbuf[prv], Rin, kx32, ky32, kz32, Fs, s32,
+                                     prev0 ? 1 : 0, bch, P);
+                    else
+                        HT3D_LAUNCH(ctx, kern, ig, ib, 0, Dbuf[cur], Dbuf[prv], Rin, kx32, ky32, kz32, Fs, s32,
+                                    prev0 ? 1 : 0, bch, P);
+                };
+                if (storef) go(k_mixed_inner<true, false>, k_mixed_inner<true, true>);
+                else go(k_mixed_inner<false, false>, k_mixed_inner<false, true>);
                 std::swap(cur, prv);
                 timer.count();
             }
