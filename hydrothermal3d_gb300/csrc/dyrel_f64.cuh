@@ -9,12 +9,13 @@
 // after row without gaps, and marches through a chunk of planes.  A thread
 // evaluates its cells' west and south fluxes and leaves them in shared memory
 // for the pair to the west and the row to the south; the z flux stays in a
-// register.  (Small grids: one cell per thread.)  What is left are 9 operations for the fluxes (15 in k_dyrel_iter),
-// 9 or 11 for their sum, 3 for the quotient (9) and 5 for the update, and one
-// more face at the block's end, at a wall and at a chunk's first plane.
+// register.  (Small grids: one cell per thread.)  What is left are 9 operations for
+// the fluxes (15 in k_dyrel_iter), 9 or 11 for their sum, 3 for the quotient (9)
+// and 5 for the update, and one more face at the block's end, at a wall and at a
+// chunk's first plane.
 //
-// us per iteration, k_dyrel_iter and this kernel: 31 x 29 x 33 8.5 -> 4.9, 63^3
-// 31.0 -> 20.6, 95^3 82 -> 58.5, 127 x 119 x 131 180 -> 131, 255^3 1440 -> 1009.
+// us per iteration, k_dyrel_iter and this kernel: 31 x 29 x 33 8.5 -> 4.7, 63^3
+// 31.0 -> 18.8, 95^3 82 -> 58.2, 127 x 119 x 131 180 -> 130, 255^3 1440 -> 1009.
 // Plain launches begin on a 2 us raster; launch_after saves the wait (63^3: 22.9).
 #pragma once
 #include "dyrel_common.cuh"
