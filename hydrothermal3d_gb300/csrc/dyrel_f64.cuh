@@ -1,6 +1,7 @@
 // The FP64 pseudo-iteration of k_dyrel_iter with every face flux evaluated once
 // and the quotient by the diagonal from its reciprocal (include from
-// -fmad=false translation units: the same values as the reference's statements).
+// -fmad=false translation units).  With the reciprocals at hand the values are
+// those of the reference's statements, without them up to div_any's (fp64_div.cuh).
 //
 // Bound by the FP64 pipe, 2 results per clock and SM: at 63^3 the fields sit in
 // L2 and at 255^3 an iteration moves 0.17 of the copy rate, so only the number

@@ -6,12 +6,16 @@
 // Newton's iteration, or rounded on the host for a divisor that a launch shares)
 // and correct a y once by its exact remainder, r = a - b q with one fma, q' =
 // fma(r, y, q) (P. Markstein, "Computation of elementary functions on the IBM
-// RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990): q' is the
-// correctly rounded quotient unless a / b lies within about 2^-51 ulp of the
-// middle between two doubles, which one pair of operands in 10^15 does; there
-// it may be the other neighbour.  Operands outside the range in which nothing
-// over- or underflows on the way (zero, infinite and NaN among them) are
-// divided by the operator.
+// RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990).  Where y is the
+// correctly rounded 1 / b (div_known, Divisor) q' is the operator's quotient
+// (every pair of operands at 6 to 11 bits of significand checked).  Newton's y
+// may be the neighbour of that.  It is for a divisor whose significand is all
+// ones, which the operator takes; for others q' may then be the other one of the
+// two doubles around a quotient that lies nearly in their middle (one pair in
+// about 2^p at p bits, 10^16 for a double).  Operands outside the range in which
+// nothing over- or underflows on the way (infinite, NaN, a zero divisor and -0,
+// of which the remainder would lose the sign, among them) are divided by the
+// operator.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -19,10 +23,8 @@
 __device__ __forceinline__ bool mid_range(double x) {
     return ((unsigned)__double2hiint(x) & 0x7fffffffu) - 0x26f00000u < 0x32000000u;
 }
-// ... or 0, as a dividend
-__device__ __forceinline__ bool mid_range0(double x) {
-    return mid_range(x) || (((unsigned)__double2hiint(x) & 0x7fffffffu) | (unsigned)__double2loint(x)) == 0u;
-}
+// ... or +0, as a dividend
+__device__ __forceinline__ bool mid_range0(double x) { return mid_range(x) || __double_as_longlong(x) == 0; }
 // 1/b to about an ulp: the hardware's approximation (20 bits or more), refined
 // to third order: y (1 + e + e^2), e = 1 - b y
 __device__ __forceinline__ double rcp_newton(double b) {
@@ -36,9 +38,12 @@ __device__ __forceinline__ double div_by(double a, double b, double y) {
     const double q = __dmul_rn(a, y);
     return __fma_rn(__fma_rn(-b, q, a), y, q);
 }
+__device__ __forceinline__ bool all_ones(double b) {
+    return __double2loint(b) == -1 && (__double2hiint(b) | 0xfff00000) == -1;
+}
 // a / b for any operands
 __device__ __forceinline__ double div_any(double a, double b) {
-    if (mid_range0(a) && mid_range(b)) return div_by(a, b, rcp_newton(b));
+    if (mid_range0(a) && mid_range(b) && !all_ones(b)) return div_by(a, b, rcp_newton(b));
     return __ddiv_rn(a, b);
 }
 // a / b where y = 1/b is at hand

@@ -8,10 +8,11 @@
 namespace {
 
 // ----------------------------------------------------------------- WENO core
-// dFdx_Weno5! body, tools/Weno5_Routines.jl:51-66 (FP64, the reference's value).
+// dFdx_Weno5! body, tools/Weno5_Routines.jl:51-66 (FP64, the reference's value but
+// for the rare quotients of fp64_div.cuh's Newton form).
 //
 // Bound by the FP64 pipe, so what counts is the number of FP64 operations: 95
-// here instead of about 165 as the statements stand, with the same results.
+// here instead of about 165 as the statements stand.
 // A product with a power of two is exact and is taken into an fma; v/6 is half
 // of v/3; max(v^2) is the square of the largest magnitude (integer compares);
 // the quotients by 3 take two operations, the others six, and the three with the

@@ -154,3 +154,26 @@ def test_fused_sweep_with_two_inflow_sides(ctx, orc, n, flow, variant):
     api.weno5_advect(ctx, Td, *[ht.from_numpy(v) for v in V], dt, *h, types, vals, variant, abi.FP64)
     inner = (slice(1, -1),) * 3
     np.testing.assert_array_equal(ht.to_numpy(Td)[inner], To[inner])
+
+
+def test_quotients_have_the_operators_bits(ctx):
+    """Init_vel_dim divides a flux by a mean of four equal densities: every pair of
+    signed zeros, ends of the fast form's range, subnormal, infinite and NaN
+    operands and some in between, compared bit by bit with the host's quotient."""
+    rng = np.random.default_rng(31)
+    ends = [0.0, 5e-324, 2.0 ** -1022, 2.0 ** -1000, np.nextafter(2.0 ** -400, 0), 2.0 ** -400, 0.1, 1.0, 3.0,
+            np.nextafter(2.0 ** 400, 0), 2.0 ** 400, 2.0 ** 1000, np.inf, np.nan]
+    v = np.array([s * e for e in ends for s in (1, -1)] + list(rng.uniform(-2, 2, 60) * 10.0 ** rng.uniform(-90, 90, 60)))
+    a, b = (m.ravel() for m in np.meshgrid(v, v))
+    n = a.size - 1
+    qx, rfv = np.zeros((n + 1, 1, 1), order="F"), np.zeros((n + 1, 2, 2), order="F")
+    qx[:, 0, 0] = a
+    rfv[:] = b[:, None, None]
+    V = [ht.zeros(n + 1, 1, 1), ht.zeros(n, 2, 1), ht.zeros(n, 1, 2)]
+    api.Init_vel_dim(ctx, *V, ht.from_numpy(qx), ht.zeros(n, 2, 1), ht.zeros(n, 1, 2), ht.from_numpy(rfv))
+    with np.errstate(all="ignore"):
+        ref = a / ((b + b + b + b) * 0.25)
+    got = ht.to_numpy(V[0])[:, 0, 0]
+    num = ~np.isnan(ref)
+    np.testing.assert_array_equal(np.isnan(got), ~num)
+    np.testing.assert_array_equal(got[num].view(np.int64), ref[num].view(np.int64))
