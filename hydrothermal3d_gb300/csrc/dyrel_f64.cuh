@@ -177,7 +177,9 @@ struct F64Launch {
     dim3 grid;
     long long blocks() const { return (long long)grid.x * grid.z; }
 };
+// (a grid has at most 65535 blocks in z: longer columns take more planes a block)
 inline F64Launch f64_shape(int cells, int threads, int zchunk, int nx, int ny, int nz) {
+    zchunk = std::max(zchunk, (nz + 65534) / 65535);
     const long long runs = (long long)((nx + cells - 1) / cells) * ny;
     return F64Launch{cells, threads, zchunk,
                      dim3((unsigned)((runs + threads - 1) / threads), 1, (unsigned)((nz + zchunk - 1) / zchunk))};

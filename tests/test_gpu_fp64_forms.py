@@ -177,3 +177,30 @@ def test_quotients_have_the_operators_bits(ctx):
     num = ~np.isnan(ref)
     np.testing.assert_array_equal(np.isnan(got), ~num)
     np.testing.assert_array_equal(got[num].view(np.int64), ref[num].view(np.int64))
+
+
+# more planes than a grid has blocks in z, a cell and three in each
+@pytest.mark.parametrize("n", [(1, 1, 100000), (3, 1, 66000)])
+def test_fp64_iteration_on_columns_of_many_planes(ctx, n):
+    """ht3d_dyrel_iterate and ht3d_dyrel_iterate_noalloc take such columns, an even
+    number of iterations of them, and equal the per-cell layout."""
+    nx, ny, nz = n
+    out = []
+    for form in ("cell", "default", "noalloc"):
+        ctx.set_tuning(abi.TUNE_DYREL_VARIANT, abi.DYREL_CELL if form == "cell" else 0)
+        rng = np.random.default_rng(37)
+        f = lambda *s: ht.from_numpy(np.asfortranarray(rng.uniform(0.5, 1.5, s)))
+        X, R, PC, F0 = f(nx + 2, ny + 2, nz + 2), f(*n), f(*n), f(*n)
+        k = [f(nx + 1, ny, nz), f(nx, ny + 1, nz), f(nx, ny, nz + 1)]
+        args = (X.data_ptr(), R.data_ptr(), *[a.data_ptr() for a in k], PC.data_ptr(), F0.data_ptr(), 3.0, 1.0, 1.0, 1.0,
+                abi.int6(0, 1, 1, 0, 0, 1), abi.dbl6(0, .5, 1, 0, 0, .2), 0.9, 0.02, 0.01, 2, *n)
+        if form == "noalloc":
+            assert ctx.lib.ht3d_dyrel_iterate_noalloc(*args, ctx.stream) == abi.OK
+            ctx.synchronize()
+        else:
+            ctx.call("ht3d_dyrel_iterate", *args)
+        out.append((ht.to_numpy(X), ht.to_numpy(F0)))
+    ctx.set_tuning(abi.TUNE_DYREL_VARIANT, 0)
+    for o in out[1:]:
+        for a, b in zip(out[0], o):
+            np.testing.assert_array_equal(a, b)
