@@ -24,7 +24,7 @@ __device__ __forceinline__ bool mid_range(double x) {
     return ((unsigned)__double2hiint(x) & 0x7fffffffu) - 0x26f00000u < 0x32000000u;
 }
 // ... or +0, as a dividend
-__device__ __forceinline__ bool mid_range0(double x) { return mid_range(x) || __double_as_longlong(x) == 0; }
+__device__ __forceinline__ bool mid_range0(double x) { return mid_range(x) || (__double2hiint(x) | __double2loint(x)) == 0; }
 // 1/b to about an ulp: the hardware's approximation (20 bits or more), refined
 // to third order: y (1 + e + e^2), e = 1 - b y
 __device__ __forceinline__ double rcp_newton(double b) {
