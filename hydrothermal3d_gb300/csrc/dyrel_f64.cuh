@@ -46,6 +46,9 @@ __global__ void __launch_bounds__(T) k_dyrel_f64(const double* __restrict__ Xin,
     after_previous();
     const int np = (nx + NC - 1) / NC, tid = threadIdx.x;
     const int t = blockIdx.x * T + tid;
+    // a warp past the plane: on thin grids most of them (with two cells per thread
+    // the plane is wide, and the test cost 2 % at 200 x 190 x 200)
+    if (NC == 1 && t - (tid & 31) >= np * ny) return;
     const int j = t / np, i = NC * (t - j * np);
     const bool row = j < ny;
     const int k0 = blockIdx.z * zchunk, k1 = min(nz, k0 + zchunk);
@@ -193,10 +196,14 @@ inline F64Launch f64_shape(int cells, int threads, int zchunk, int nx, int ny, i
 // planes while an SM holds its two at once (80 x 70 x 75: 31.0, 32.6 with one cell;
 // but 80^3, a second round of them: 42.1, 39.0).  From 2^19 cells on the rounds blend:
 // three planes up to 2^22 (95^3: 58.2, 63.0 with one cell; 127 x 119 x 131: 130, two
-// planes 137), eight above (255^3: 1009, three 1037).
+// planes 137), eight above (255^3: 1009, three 1037).  A plane of less than two
+// blocks of pairs is left to the small shapes, where its empty warps leave: per
+// iteration 1 x 1 x 4096 56 us with them and 17 without (k_dyrel_iter 29), 2 x 2 x
+// 60000 589 and 167 (566).
 inline F64Launch f64_launch(int sms, int nx, int ny, int nz) {
     const long long n = (long long)nx * ny * nz;
-    if (n >= (1LL << 19)) return f64_shape(2, 256, n < (1LL << 22) ? 3 : 8, nx, ny, nz);
+    const int plane = nx * ny, pairs = (nx + 1) / 2 * ny;
+    if (n >= (1LL << 19) && pairs >= 512) return f64_shape(2, 256, n < (1LL << 22) ? 3 : 8, nx, ny, nz);
     struct Shape { int cells, threads, planes, most, ps; };  // most: blocks that an SM may have; ps a slot
     const Shape shapes[] = {{1, 128, 1, 1 << 30, 11200}, {1, 256, 1, 1 << 30, 10800}, {2, 64, 2, 9, 9500},
                             {2, 256, 2, 2, 8800}, {2, 256, 3, 2, 8800}};
@@ -205,8 +212,9 @@ inline F64Launch f64_launch(int sms, int nx, int ny, int nz) {
     for (const Shape& h : shapes) {
         const F64Launch L = f64_shape(h.cells, h.threads, h.planes, nx, ny, nz);
         const long long share = (L.blocks() + sms - 1) / sms;
-        if (share > h.most) continue;
-        const long long cost = share * h.cells * h.threads * h.planes * h.ps + 1200000LL * h.planes;
+        if (share > h.most || (h.cells == 1 && h.threads > 128 && plane <= 128)) continue;
+        const int busy = h.cells == 1 ? std::min(h.threads, (plane + 31) / 32 * 32) : h.threads;
+        const long long cost = share * h.cells * busy * h.planes * h.ps + 1200000LL * h.planes;
         if (least < 0 || cost < least) least = cost, best = L;
     }
     return best;

@@ -179,8 +179,9 @@ def test_quotients_have_the_operators_bits(ctx):
     np.testing.assert_array_equal(got[num].view(np.int64), ref[num].view(np.int64))
 
 
-# more planes than a grid has blocks in z, a cell and three in each
-@pytest.mark.parametrize("n", [(1, 1, 100000), (3, 1, 66000)])
+# more planes than a grid has blocks in z, a cell and three in each; warps past a thin
+# plane in blocks of 128 and 256, also where the grid has many cells
+@pytest.mark.parametrize("n", [(1, 1, 100000), (3, 1, 66000), (5, 7, 40), (13, 11, 50), (20, 13, 2100)])
 def test_fp64_iteration_on_columns_of_many_planes(ctx, n):
     """ht3d_dyrel_iterate and ht3d_dyrel_iterate_noalloc take such columns, an even
     number of iterations of them, and equal the per-cell layout."""
