@@ -13,6 +13,14 @@ void* ht3d_scratch(ht3d_ctx* ctx, int slot, size_t bytes) {
     }
     void* p = nullptr;
     cudaError_t e = cudaMalloc(&p, bytes);
+    if (e != cudaSuccess && slot != SLOT_SPARE && ctx->slot_ptr[SLOT_SPARE]) {
+        cudaGetLastError();
+        HT3D_CUDA(cudaStreamSynchronize(ctx->stream));
+        HT3D_CUDA(cudaFree(ctx->slot_ptr[SLOT_SPARE]));
+        ctx->slot_ptr[SLOT_SPARE] = nullptr;
+        ctx->slot_bytes[SLOT_SPARE] = 0;
+        e = cudaMalloc(&p, bytes);
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         throw ht3d_error(HT3D_ERR_NOMEM, std::string("cudaMalloc scratch failed: ") + cudaGetErrorString(e));
@@ -20,6 +28,27 @@ void* ht3d_scratch(ht3d_ctx* ctx, int slot, size_t bytes) {
     ctx->slot_ptr[slot] = p;
     ctx->slot_bytes[slot] = bytes;
     return p;
+}
+
+// Work memory that the caller can do without (taken after all that it needs), or
+// null: where the device would be left with little, and in a stream capture, whose
+// graph may be launched when a later call has let the memory go.  A call that needs
+// the memory for something else takes it back (ht3d_scratch).
+void* ht3d_scratch_spare(ht3d_ctx* ctx, size_t bytes) {
+    cudaStreamCaptureStatus capture;
+    HT3D_CUDA(cudaStreamIsCapturing(ctx->stream, &capture));
+    if (capture != cudaStreamCaptureStatusNone) return nullptr;
+    if (ctx->slot_bytes[SLOT_SPARE] < bytes) {
+        size_t left = 0, total = 0;
+        HT3D_CUDA(cudaMemGetInfo(&left, &total));
+        if (left < bytes + (256ULL << 20)) return nullptr;
+    }
+    try {
+        return ht3d_scratch(ctx, SLOT_SPARE, bytes);
+    } catch (const ht3d_error& e) {
+        if (e.code != HT3D_ERR_NOMEM) throw;
+        return nullptr;
+    }
 }
 
 void ht3d_fetch_results(ht3d_ctx* ctx, const double* d_src, int count) {

@@ -16,12 +16,12 @@ int ht3d_dyrel_solve_fp64(ht3d_ctx* ctx, double* X, const double* R, const doubl
     IterLaunch L = iter_launch(ctx, nx, ny, nz);
     const bool fixed_variant = ctx->dyrel_variant != 0;  // the caller's thread layout
     const F64Launch L64 = f64_launch(ctx->num_sms, nx, ny, nz);
-    double* iPC = fixed_variant ? nullptr : (double*)ht3d_scratch(ctx, SLOT_G, sizeof(double) * n);
     const long long nsetup = (long long)((nx + 31) / 32) * ((ny + 7) / 8) * nz;
     // per-cell check terms (3n) followed by tree-pass work space
     const long long nwork = 3 * n + 6 * ((n + 1023) / 1024 + 1);
     double* parts = (double*)ht3d_scratch(ctx, SLOT_PARTIALS, sizeof(double) * std::max(nwork, nsetup));
     double* dres = (double*)ht3d_scratch(ctx, SLOT_RESULT, sizeof(double) * 64);
+    double* iPC = fixed_variant ? nullptr : (double*)ht3d_scratch_spare(ctx, sizeof(double) * n);
 
     BC6<double> bc;
     for (int f = 0; f < 6; ++f) {
@@ -51,10 +51,10 @@ int ht3d_dyrel_solve_fp64(ht3d_ctx* ctx, double* X, const double* R, const doubl
     // the plain, storing and checking iterations
     F64Kernel<0>::Fn kern64[3];
     size_t smem64[3] = {0, 0, 0};
-    if (iPC) {
-        kern64[0] = F64Kernel<MODE_PLAIN>::get(cX != 0.0, true, L64);
-        kern64[1] = F64Kernel<MODE_STOREF>::get(cX != 0.0, true, L64);
-        kern64[2] = F64Kernel<MODE_CHECK>::get(cX != 0.0, true, L64);
+    if (!fixed_variant) {
+        kern64[0] = F64Kernel<MODE_PLAIN>::get(cX != 0.0, iPC != nullptr, L64);
+        kern64[1] = F64Kernel<MODE_STOREF>::get(cX != 0.0, iPC != nullptr, L64);
+        kern64[2] = F64Kernel<MODE_CHECK>::get(cX != 0.0, iPC != nullptr, L64);
         for (int v = 0; v < 3; ++v) smem64[v] = even_smem(ctx, kern64[v], L64.threads, L64.blocks());
     }
     double* cur = X;
@@ -69,7 +69,7 @@ int ht3d_dyrel_solve_fp64(ht3d_ctx* ctx, double* X, const double* R, const doubl
         sc.h1 = S.h1;
         sc.h2 = S.h2;
         sc.dtau = S.dtau;
-        if (iPC) {
+        if (!fixed_variant) {
             const int v = chk ? 2 : (storef ? 1 : 0);
             launch_after(ctx, kern64[v], L64.grid, L64.threads, smem64[v], cur, nxt, R, kx, ky, kz, PC, iPC, F0, F,
                          DyrelScalT<double>(sc), bc, nx, ny, nz, L64.zchunk, parts);
@@ -144,10 +144,9 @@ extern "C" int ht3d_dyrel_iterate(ht3d_ctx* ctx, double* X_ex, const double* R, 
         double* X2 = (double*)ht3d_scratch(ctx, SLOT_AUX0, sizeof(double) * nex);
         // the reciprocals pay from a few iterations on (3 operations a cell each instead of 6, and 1 division here)
         double* iPC = nullptr;
-        if (n_iter >= 4) {
-            iPC = (double*)ht3d_scratch(ctx, SLOT_G, sizeof(double) * n);
+        if (n_iter >= 4) iPC = (double*)ht3d_scratch_spare(ctx, sizeof(double) * n);
+        if (iPC)
             HT3D_LAUNCH(ctx, k_reciprocal, (unsigned)std::min<long long>((n + 255) / 256, ctx->num_sms * 16LL), 256, 0, iPC, PC, n);
-        }
         const F64Launch L = f64_launch(ctx->num_sms, nx, ny, nz);
         const DyrelScalT<double> sc(DyrelScal{h1, h2, dtau, cX, 1.0 / dx, 1.0 / dy, 1.0 / dz});
         const auto kern = F64Kernel<MODE_PLAIN>::get(cX != 0.0, iPC != nullptr, L);

@@ -34,6 +34,7 @@ enum ScratchSlot {
     SLOT_ENS_SOLVE,     // batched solve: per-instance FP64 and padded FP32 fields
     SLOT_ENS_TAB,       // batched solve: per-instance check results
     SLOT_RES,           // resident iterations: face words of the blocks
+    SLOT_SPARE,         // what a call can do without (ht3d_scratch_spare)
     SLOT_ENS_STEP,      // ensemble step: per-instance residual, flux and conductivity fields
     SLOT_COUNT
 };
@@ -123,6 +124,7 @@ static inline int ht3d_guard(ht3d_ctx* ctx, Fn&& body, bool sync = true) {
 }
 
 void* ht3d_scratch(ht3d_ctx* ctx, int slot, size_t bytes);
+void* ht3d_scratch_spare(ht3d_ctx* ctx, size_t bytes);
 
 // every pointer argument is set (entry points reject NULL before any launch)
 template <typename... P>
