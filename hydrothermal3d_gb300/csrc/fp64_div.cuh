@@ -39,7 +39,7 @@ __device__ __forceinline__ double div_by(double a, double b, double y) {
     return __fma_rn(__fma_rn(-b, q, a), y, q);
 }
 __device__ __forceinline__ bool all_ones(double b) {
-    return __double2loint(b) == -1 && (__double2hiint(b) | 0xfff00000) == -1;
+    return __double2loint(b) == -1 && (__double2hiint(b) & 0xfffff) == 0xfffff;
 }
 // a / b for any operands
 __device__ __forceinline__ double div_any(double a, double b) {

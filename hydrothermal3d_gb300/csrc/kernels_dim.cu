@@ -551,6 +551,10 @@ __device__ __forceinline__ double bc_value(const double* __restrict__ S, const s
     return v;
 }
 
+constexpr int kRhofTerms = 7;
+struct RhofPlanes {
+    double* p[kRhofTerms];
+};
 struct DimIterArgs {
     const double* Xin;
     double* Xout;
@@ -570,7 +574,7 @@ struct DimIterArgs {
     // Darcy
     const double* prf0;    // ϕρf_old
     const double* rfy;     // av_xza(ρfv) on y faces
-    const double* tt;      // the density's temperature terms (k_rhof_terms)
+    RhofPlanes tt;         // the density's temperature terms (k_rhof_terms)
 };
 
 struct DimScal {
@@ -581,18 +585,19 @@ struct DimScal {
 };
 
 // Terms of law_rhof_C that depend on the temperature alone, which does not
-// change during a Darcy solve, in planes of n cells: T, T^2, T^3 (in C) and the
-// polynomial's own T, T^2, T^3 and T^4 terms.
-constexpr int kRhofTerms = 7;
-__global__ void k_rhof_terms(double* __restrict__ tt, const double* __restrict__ Tex, double s_T, int nx, int ny, int nz) {
-    const long long n = (long long)nx * ny * nz;
+// change during a Darcy solve: T, T^2, T^3 (in C) and the polynomial's own T, T^2,
+// T^3 and T^4 terms.  They take no memory of their own: four lie in fields that the
+// solve has done with, and the first three where a check leaves its per-cell terms,
+// after which they are written again (AGAIN: those alone).
+template <bool AGAIN>
+__global__ void k_rhof_terms(RhofPlanes tt, const double* __restrict__ Tex, double s_T, int nx, int ny, int nz) {
     for_cells_z(nx, ny, nz, [&](int i, int j, int k) {
         const long long c = CI(i, j, k);
         const double T_C = Tex[EXI(i + 1, j + 1, k + 1)] * s_T - 273.15;
         const double T2 = T_C * T_C, T3 = T_C * T_C * T_C, T4 = T2 * T2;
         const double v[kRhofTerms] = {T_C, T2, T3, -0.3922 * T_C, -0.003774 * T2, 2.955e-6 * T3, 5.698e-11 * T4};
 #pragma unroll
-        for (int q = 0; q < kRhofTerms; ++q) tt[c + q * n] = v[q];
+        for (int q = 0; q < (AGAIN ? 3 : kRhofTerms); ++q) tt.p[q][c] = v[q];
     });
 }
 // law_rhof_C (laws.cuh), statement for statement, with those terms at hand
@@ -705,6 +710,12 @@ __global__ void __launch_bounds__(T) k_dim_iter(DimIterArgs A, DimScal s, DimBC 
 #pragma unroll
             for (int m = 0; m < NC; ++m) qN[m] = south[par][m][tid + np];
         }
+        double tt[NC][kRhofTerms];  // both cells' before either's arithmetic
+        if (PRESSURE && TRANS)
+#pragma unroll
+            for (int m = 0; m < NC; ++m)
+#pragma unroll
+                for (int r = 0; r < kRhofTerms; ++r) tt[m][r] = A.tt.p[r][c + off(m)];
 #pragma unroll
         for (int m = 0; m < NC; ++m) {
             const int cc = c + off(m), p = A.ph[e + off(m)];
@@ -712,10 +723,7 @@ __global__ void __launch_bounds__(T) k_dim_iter(DimIterArgs A, DimScal s, DimBC 
             if (PRESSURE) {
                 if (TRANS) {
                     // ϕρf from the pre-boundary-kernel pressure (the reference runs ϕρf first)
-                    double tt[kRhofTerms];
-#pragma unroll
-                    for (int r = 0; r < kRhofTerms; ++r) tt[r] = A.tt[cc + r * n];
-                    const double rho = rhof_from_terms(tt, A.Xin[e + off(m)] * s.s_sigma);
+                    const double rho = rhof_from_terms(tt[m], A.Xin[e + off(m)] * s.s_sigma);
                     const double prf = div_known((p == 2 ? s.phi_f : s.phi_i) * rho, s.s_rho, s.y_rho);
                     f = s.tdt * (prf - A.prf0[cc]);
                 }
@@ -801,7 +809,6 @@ inline F64Launch dim_launch(int nx, int ny, int nz) {
 
 struct DimWork {
     double *X2, *kv, *dumc, *kx, *ky, *kz, *rC, *PC, *G, *F, *F0, *T0, *P0, *rfy, *terms, *prf0;
-    double *iPC, *tt;   // 1 / PC; the Darcy iteration's temperature terms, or the heat's rhoC factor
     const double* Tex;  // temperature (ex) read by the Darcy iteration
     signed char* ph;
 };
@@ -824,10 +831,19 @@ int dim_dyrel(ht3d_ctx* ctx, double* X, DimWork& W, const double* wN, DimScal s,
     s.phi_f = 3 * s.phi_i;
     s.y_rho = 1.0 / s.s_rho;
     const unsigned g1 = (unsigned)std::max<long long>(1, std::min<long long>((n + 255) / 256, ctx->num_sms * 16LL));
-    HT3D_LAUNCH(ctx, k_reciprocal, g1, 256, 0, W.iPC, W.PC, n);
+    double* const iPC = W.dumc;  // free: the conductivities are smoothed
+    HT3D_LAUNCH(ctx, k_reciprocal, g1, 256, 0, iPC, W.PC, n);
     const bool trans = s.tdt != 0.0;
-    if (!PRESSURE) HT3D_LAUNCH(ctx, k_scale_rc, g1, 256, 0, W.tt, W.rC, s.transient, s._dt, n);
-    else if (trans) HT3D_LAUNCH(ctx, k_rhof_terms, grid3z(nx, ny, nz), kBlock3, 0, W.tt, W.Tex, s.s_T, nx, ny, nz);
+    // kv is free: the heat's conductivities, or the density on the faces, are formed
+    double* const rCt = W.kv;
+    RhofPlanes tt{};
+    const dim3 gt = grid3z(nx, ny, nz);
+    if (!PRESSURE) HT3D_LAUNCH(ctx, k_scale_rc, g1, 256, 0, rCt, W.rC, s.transient, s._dt, n);
+    else if (trans) {
+        // rC, T0 and P0 went into PC and prf0
+        tt = RhofPlanes{{W.terms, W.terms + n, W.terms + 2 * n, W.kv, W.rC, W.T0, W.P0}};
+        HT3D_LAUNCH(ctx, k_rhof_terms<false>, gt, kBlock3, 0, tt, W.Tex, s.s_T, nx, ny, nz);
+    }
     const F64Launch L = dim_launch(nx, ny, nz);
     const int cb = (int)L.grid.x, wb = (int)(cb * L.grid.z);
     const unsigned grd = (unsigned)(wb + shell_blocks(L.threads, nx, ny, nz));
@@ -850,8 +866,8 @@ int dim_dyrel(ht3d_ctx* ctx, double* X, DimWork& W, const double* wN, DimScal s,
     size_t smem[3];
     for (int v = 0; v < 3; ++v) smem[v] = even_smem(ctx, kern[v], L.threads, wb);
     DimIterArgs A;
-    A.ph = W.ph; A.wN = wN; A.kx = W.kx; A.ky = W.ky; A.kz = W.kz; A.PC = W.PC; A.iPC = W.iPC; A.F0 = W.F0; A.F = W.F;
-    A.terms = W.terms; A.T0 = W.T0; A.rCt = W.tt; A.tt = W.tt; A.prf0 = W.prf0; A.rfy = W.rfy;
+    A.ph = W.ph; A.wN = wN; A.kx = W.kx; A.ky = W.ky; A.kz = W.kz; A.PC = W.PC; A.iPC = iPC; A.F0 = W.F0; A.F = W.F;
+    A.terms = W.terms; A.T0 = W.T0; A.rCt = rCt; A.tt = tt; A.prf0 = W.prf0; A.rfy = W.rfy;
     double* cur = X;
     double* nxt = W.X2;
     DyrelCheck C;
@@ -868,6 +884,8 @@ int dim_dyrel(ht3d_ctx* ctx, double* X, DimWork& W, const double* wN, DimScal s,
         if (chk) {
             tree_sum3(ctx, W.terms, n, W.terms + 3 * n);
             if (C.update(S, prm, ctx->h_result[0], ctx->h_result[1], ctx->h_result[2], (double)n, iter, true)) break;
+            if (PRESSURE && trans && iter < prm->nitmax)
+                HT3D_LAUNCH(ctx, k_rhof_terms<true>, gt, kBlock3, 0, tt, W.Tex, s.s_T, nx, ny, nz);
         }
     }
     if (cur != X) HT3D_CUDA(cudaMemcpyAsync(X, cur, sizeof(double) * nex, cudaMemcpyDeviceToDevice, ctx->stream));
@@ -911,8 +929,6 @@ extern "C" int ht3d_step_v18(ht3d_ctx* ctx, double* Tc_ex, double* Pc_ex, const 
         W.rfy = (double*)ht3d_scratch(ctx, SLOT_STEP_TY, sizeof(double) * nfy);
         W.terms = (double*)ht3d_scratch(ctx, SLOT_PARTIALS, sizeof(double) * (3 * n + 6 * ((n + 1023) / 1024 + 1)));
         W.ph = (signed char*)ht3d_scratch(ctx, SLOT_AUX2, nex);
-        W.iPC = (double*)ht3d_scratch(ctx, SLOT_AUX3, sizeof(double) * (1 + kRhofTerms) * n);
-        W.tt = W.iPC + n;
         const double dx = p->dx, dy = p->dy, dz = p->dz, _dx = 1.0 / dx, _dy = 1.0 / dy, _dz = 1.0 / dz;
         const double dt = p->dt, _dt = 1.0 / dt, transient = p->it == 0 ? 0.0 : 1.0;
         const dim3 gv = grid3(nx + 1, ny + 1, nz + 1, kBlock3), gc = grid3(nx, ny, nz, kBlock3);

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import hydrothermal3d_gb300 as ht
-from hydrothermal3d_gb300 import api, abi
+from hydrothermal3d_gb300 import api, abi, v18
 
 pytestmark = pytest.mark.gpu
 TYPES, VALS = (0, 1, 1, 0, 0, 1), (0.0, 0.5, 1.0, 0.0, 0.0, 0.2)
@@ -105,3 +105,29 @@ def test_iterations_captured_after_a_shorter_call(gpu_stream):
     gpu_stream.synchronize()
     assert torch.equal(d["X"], ref[0]) and torch.equal(d["F0"], ref[1])
     c.close()
+
+
+def test_dimensional_step_takes_no_memory_beyond_its_fields(fresh):
+    """Its work memory: a ghosted field and one of phase codes, the vertex and face
+    conductivities and the faces' density, eight cell fields and a check's three
+    terms a cell (the reciprocals and the density's temperature terms lie in fields
+    that are done with); 2 MB of rounding for each of the eighteen allocations (no
+    advection)."""
+    n = nx, ny, nz = 128, 120, 100
+    b = v18.box(*n, seed=3, nitout=2, nitmax=5)
+    b["params"].it, b["params"].advection = 2, 0
+    d = [ht.from_numpy(b[k]) for k in ("T", "P", "phc", "phv", "wN", "kmul")]
+    V = [ht.zeros(nx + 1, ny, nz), ht.zeros(nx, ny + 1, nz), ht.zeros(nx, ny, nz + 1)]
+    small = v18.box(8, 8, 8, seed=3, nitout=2, nitmax=5)
+    small["params"].it, small["params"].advection = 2, 0
+    c = ht.Context(device=0, stream=fresh.stream)  # loads the kernels
+    api.step_v18(c, *[ht.from_numpy(small[k]) for k in ("T", "P", "phc", "phv", "wN", "kmul")], ht.zeros(9, 8, 8),
+                 ht.zeros(8, 9, 8), ht.zeros(8, 8, 9), small["params"])
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    api.step_v18(fresh, *d, *V, b["params"])
+    used = before - torch.cuda.mem_get_info()[0]
+    c.close()
+    cells, ghosted, vertices = nx * ny * nz, (nx + 2) * (ny + 2) * (nz + 2), (nx + 1) * (ny + 1) * (nz + 1)
+    faces = sum(v.numel() for v in V) + V[1].numel()
+    assert used <= 8 * (ghosted + vertices + faces + 11 * cells) + ghosted + 18 * (2 << 20)
