@@ -1190,7 +1190,9 @@ int ht3d_dyrel_solve_mixed(ht3d_ctx* ctx, double* X, const double* R, const doub
     sc._dy = 1.0 / dy;
     sc._dz = 1.0 / dz;
     const dim3 ib(HT3D_MIX_BS), ig((unsigned)(((long long)P.nq * ny + HT3D_MIX_BS - 1) / HT3D_MIX_BS), (unsigned)nz);
-    // up to three and a half waves of k_mixed_inner (127^3 8.3 us after, 9.5 plain; 133^3 10.6 and 9.9)
+    // up to three and a half waves of k_mixed_inner (127^3 8.3 us after, 9.5 plain; 133^3 10.6 and 9.9),
+    // but plain behind a check, for whose sums the host waits: nothing to hide there, and a dependent
+    // launch on an idle stream starts later (16^3, a check every second iteration: 34 us a pair, 36)
     const bool single_after = (long long)ig.x * ig.y <= 56LL * ctx->num_sms;
     // two iterations per pass (k_mixed_inner2) inside runs of inner iterations
     bool pairs = want_pairs;
@@ -1296,7 +1298,7 @@ int ht3d_dyrel_solve_mixed(ht3d_ctx* ctx, double* X, const double* R, const doub
             const int left = pair_end - iter + 1;
             // (an iteration that has to leave F goes by itself)
             const int res_end = run_end - (run_end == nmax || is_check(run_end + 1, prm->nitout) ? 1 : 0);
-            if (resident && res_end > iter && dtau_prev == sc.dtau) {
+            if (resident && res_end - iter + 1 >= res_shortest(plan) && dtau_prev == sc.dtau) {
                 resident = run_resident(iter, res_end, s32, prev0, cur, prv);
                 ctx->res_off = !resident;
                 if (resident) {
@@ -1332,7 +1334,7 @@ int ht3d_dyrel_solve_mixed(ht3d_ctx* ctx, double* X, const double* R, const doub
                 ++iter;  // the pass did iterations iter and iter + 1
             } else {
                 auto go = [&](auto kern, auto kern_after) {
-                    if (single_after)
+                    if (single_after && !last_chk)
                         launch_after(ctx, kern_after, ig, ib, 0, Dbuf[cur], Dbuf[prv], Rin, kx32, ky32, kz32, Fs, s32,
                                      prev0 ? 1 : 0, bch, P);
                     else

@@ -514,6 +514,12 @@ inline ResPlan res_plan_full(const Pad& P, int sms) {
     }
     return ResPlan();
 }
+// The shortest run of a solve that pays for loading a block's fields and writing
+// them back.  300 iterations, runs of two with a check behind each in one launch
+// and single: 16^3 3.38 and 2.99 ms, 95^3 (five planes) 9.24 and 8.93, 127 x 119 x
+// 131 15.9 and 15.7; of four 2.32 and 2.31, 6.83 and 6.46, 11.4 and 11.6; of six 1.79
+// and 1.89, 5.29 and 5.33, 9.09 and 9.35.
+inline int res_shortest(const ResPlan& r) { return r.bz == 5 ? 6 : 4; }
 inline size_t res_words(const ResPlan& r) { return (size_t)r.ctas() * 8 * res_faces(r.bz, r.nq, r.T); }
 
 // Face words of a launch: numbers of earlier iterations may stand in them, so
