@@ -25,15 +25,18 @@ namespace {
 // launch_after, six to a sweep.  Blocks of 32 x 8 cells, plain launches and
 // second derivatives by the whole warp before, in a rough flow: 48 x 48 x 24 180 us
 // of kernels, now 126 with the gaps between them; 127^3, smooth, 3.40 -> 3.07 ms.
-template <int AXIS, int QUIRK, int STAGE, int PREC, int T>
+// TILE: 32 x T / 32 cells per block, for the mixed form where rows fill them.
+template <int AXIS, int QUIRK, int STAGE, int PREC, int T, bool TILE>
 __global__ void __launch_bounds__(T) k_weno_stage(const double* __restrict__ src, double* dst, const double* T0,
                                                   const double* __restrict__ V, double dt, double h, WenoBC bc, int nx,
                                                   int ny, int nz) {
     after_previous();
-    const int tid = threadIdx.x, k = blockIdx.y;
-    const int c = blockIdx.x * T + tid, j0 = c / nx;
-    const bool live = j0 < ny;
-    const int j = live ? j0 : ny - 1, i = live ? c - j0 * nx : nx - 1;  // threads past the plane store nothing
+    const int tid = threadIdx.x, k = TILE ? blockIdx.z : blockIdx.y;
+    const int c = blockIdx.x * T + tid, j0 = TILE ? blockIdx.y * (T / 32) + tid / 32 : c / nx;
+    const int i0 = TILE ? blockIdx.x * 32 + tid % 32 : c - j0 * nx;
+    const bool live = j0 < ny && (!TILE || i0 < nx);
+    if (TILE && !live) return;
+    const int j = live ? j0 : ny - 1, i = live ? i0 : nx - 1;  // threads past the plane store nothing
     const int n1 = nx + 2, n2 = ny + 2;
     const long long e = (i + 1) + (long long)n1 * ((j + 1) + (long long)n2 * (k + 1));
     const int idx = AXIS == 0 ? i : (AXIS == 1 ? j : k);
@@ -258,19 +261,29 @@ void weno_axis(ht3d_ctx* ctx, double* T0, double* T1, const double* V, double dt
     // Short blocks spread a small grid evenly over the SMs (sweep at 48 x 48 x 24: 113
     // us, 139 with 256 threads), long ones fill the queue's warps better (127^3, rough
     // flow: 3.58 ms, 3.69 with 128).
-    auto go = [&](auto threads) {
+    auto go = [&](auto threads, auto tile) {
         constexpr int T = decltype(threads)::value;
-        const dim3 g((unsigned)(((long long)nx * ny + T - 1) / T), nz);
-        const long long blocks = (long long)g.x * g.y;
-        launch_after(ctx, k_weno_stage<AXIS, QUIRK, 1, PREC, T>, g, T,
-                     even_smem(ctx, k_weno_stage<AXIS, QUIRK, 1, PREC, T>, T, blocks), T0, T1, (const double*)nullptr, V,
+        constexpr bool TILE = decltype(tile)::value;
+        const dim3 g = TILE ? dim3((nx + 31) / 32, (ny + T / 32 - 1) / (T / 32), nz)
+                            : dim3((unsigned)(((long long)nx * ny + T - 1) / T), nz);
+        const long long blocks = (long long)g.x * g.y * g.z;
+        launch_after(ctx, k_weno_stage<AXIS, QUIRK, 1, PREC, T, TILE>, g, T,
+                     even_smem(ctx, k_weno_stage<AXIS, QUIRK, 1, PREC, T, TILE>, T, blocks), T0, T1, (const double*)nullptr, V,
                      dt, h, bc, nx, ny, nz);
-        launch_after(ctx, k_weno_stage<AXIS, QUIRK, 2, PREC, T>, g, T,
-                     even_smem(ctx, k_weno_stage<AXIS, QUIRK, 2, PREC, T>, T, blocks), T1, T0, T0, V, dt, h, bc, nx, ny,
+        launch_after(ctx, k_weno_stage<AXIS, QUIRK, 2, PREC, T, TILE>, g, T,
+                     even_smem(ctx, k_weno_stage<AXIS, QUIRK, 2, PREC, T, TILE>, T, blocks), T1, T0, T0, V, dt, h, bc, nx, ny,
                      nz);
     };
-    if ((long long)nx * ny * nz < (1LL << 17)) go(std::integral_constant<int, 128>());
-    else go(std::integral_constant<int, 256>());
+    // The mixed form is not bound by the FP64 pipe alone: from 2^19 cells on, tiles win
+    // where hardly a lane of them is idle (periodic sweep, tiles and runs: 95^3 632 and
+    // 646 us, 190 x 255 x 200 5.59 and 5.70 ms, 255^3 9.08 and 9.26; but 63^3 255 and
+    // 245 us, 130 x 140 x 120 1.63 and 1.46 ms).
+    const long long n = (long long)nx * ny * nz;
+    constexpr std::integral_constant<int, 256> t256;
+    if (n < (1LL << 17)) return go(std::integral_constant<int, 128>(), std::false_type());
+    if constexpr (PREC != 0)
+        if (n >= (1LL << 19) && (nx + 31) / 32 * 32 - nx <= nx / 48) return go(t256, std::true_type());
+    go(t256, std::false_type());
 }
 
 template <int QUIRK, int PREC>
