@@ -1227,9 +1227,9 @@ int ht3d_dyrel_solve_mixed(ht3d_ctx* ctx, double* X, const double* R, const doub
     // runs of inner iterations in one launch, where the grid fits the chip and
     // the caller left the iteration to the library (a batched tile shape or a
     // temporal setting of their own means the kernels that these select)
-    const bool may_reside = ctx->mixed_temporal == 1 && !ctx->ens_tile && !ctx->ens_block && !ctx->res_off;
+    const bool may_reside = ctx->mixed_temporal == 1 && !ctx->ens_tile && !ctx->ens_block;
     const ResPlan plan = may_reside && !pairs ? res_plan(P, ctx->num_sms) : ResPlan();
-    bool resident = plan.bz > 0;
+    const bool resident = res_fits(ctx, plan) && res_reserve(ctx, res_words(plan));
     if (resident) {
         derr = (int*)ht3d_scratch(ctx, SLOT_AUX0, sizeof(int) * 16);
         HT3D_CUDA(cudaMemsetAsync(derr, 0, sizeof(int), ctx->stream));
@@ -1246,9 +1246,9 @@ int ht3d_dyrel_solve_mixed(ht3d_ctx* ctx, double* X, const double* R, const doub
         L.err = derr;
         L.block0[0] = 0;
         L.block0[1] = plan.ctas();
-        u64* x = res_exchange(ctx, res_words(plan), L.iters, L.tag);
+        u64* x = res_exchange(ctx, L.iters, L.tag);
         L.rec[0] = res_member(plan, P, Dbuf[cur], Dbuf[prv], Rin, kx32, ky32, kz32, Dbuf[cur], Dbuf[prv], s32, bch, x);
-        return res_launch(ctx, plan.bz, L, plan.T, res_smem(plan.bz, plan.nq, plan.by));
+        res_launch(ctx, plan.bz, L, plan.T, res_smem(plan.bz, plan.nq, plan.by));
     };
     InnerTimer timer(ctx);
     double* xcur = X;
@@ -1299,15 +1299,12 @@ int ht3d_dyrel_solve_mixed(ht3d_ctx* ctx, double* X, const double* R, const doub
             // (an iteration that has to leave F goes by itself)
             const int res_end = run_end - (run_end == nmax || is_check(run_end + 1, prm->nitout) ? 1 : 0);
             if (resident && res_end - iter + 1 >= res_shortest(plan) && dtau_prev == sc.dtau) {
-                resident = run_resident(iter, res_end, s32, prev0, cur, prv);
-                ctx->res_off = !resident;
-                if (resident) {
-                    timer.count(res_end - iter + 1);
-                    prev0 = false;
-                    it_done = iter = res_end;
-                    last_fp64 = last_chk = false;
-                    continue;
-                }
+                run_resident(iter, res_end, s32, prev0, cur, prv);
+                timer.count(res_end - iter + 1);
+                prev0 = false;
+                it_done = iter = res_end;
+                last_fp64 = last_chk = false;
+                continue;
             }
             // a pass starts only on a steady iteration (Dprev stored, mom = h1)
             if (pairs && !prev0 && dtau_prev == sc.dtau && left >= 2 && left % 2 == 0) {
@@ -1694,11 +1691,14 @@ void ht3d_ensemble_solve_mixed(ht3d_ctx* ctx, EnsSolveInst* in, int n) {
     // ---- runs of inner iterations in one launch per wave of members that fit
     // the chip together (unless the caller chose a tile shape)
     std::vector<ResPlan> plans(n);
-    bool resident = !ctx->ens_tile && !ctx->ens_block && !ctx->res_off && ctx->mixed_temporal == 1;
+    bool resident = !ctx->ens_tile && !ctx->ens_block && ctx->mixed_temporal == 1;
+    size_t cta_words = 0;  // face words of a CTA at most
     for (int q : order) {
         if (resident) plans[q] = res_plan_full(H[q].P, ctx->num_sms);
-        resident = resident && plans[q].bz;
+        resident = resident && res_fits(ctx, plans[q]);
+        cta_words = std::max(cta_words, resident ? res_words(plans[q]) / plans[q].ctas() : 0);
     }
+    resident = resident && res_reserve(ctx, cta_words * ctx->num_sms);
     int* derr = nullptr;
     if (resident) {
         tuning = false;
@@ -1716,7 +1716,6 @@ void ht3d_ensemble_solve_mixed(ht3d_ctx* ctx, EnsSolveInst* in, int n) {
         std::stable_sort(left.begin(), left.end(), [&](int a, int b) {
             return plans[a].bz != plans[b].bz ? plans[a].bz > plans[b].bz : plans[a].ctas() > plans[b].ctas();
         });
-        bool first = true;
         while (!left.empty()) {
             ResLaunch L;
             L.n = 0;
@@ -1728,7 +1727,7 @@ void ht3d_ensemble_solve_mixed(ht3d_ctx* ctx, EnsSolveInst* in, int n) {
             L.block0[0] = 0;
             const int bz = plans[left[0]].bz, cap = ctx->num_sms;
             std::vector<int> wave, rest;
-            size_t words = 0, smem = 0;
+            size_t smem = 0;
             int threads = 0;
             for (int q : left) {
                 const ResPlan& p = plans[q];
@@ -1739,25 +1738,19 @@ void ht3d_ensemble_solve_mixed(ht3d_ctx* ctx, EnsSolveInst* in, int n) {
                 wave.push_back(q);
                 L.block0[L.n + 1] = L.block0[L.n] + p.ctas();
                 ++L.n;
-                words += res_words(p);
                 smem = std::max(smem, res_smem(p.bz, p.nq, p.by));
                 threads = std::max(threads, p.T);
             }
-            u64* x = res_exchange(ctx, words, iters, L.tag);
+            u64* x = res_exchange(ctx, iters, L.tag);
             for (int m = 0; m < L.n; ++m) {
                 EnsHost& h = H[wave[m]];
                 L.rec[m] = res_member(plans[wave[m]], h.P, h.f32[parity], h.f32[parity ^ 1], h.f32[3], h.f32[4], h.f32[5],
                                       h.f32[6], h.f32[to], h.f32[to ^ 1], mix_scal(h.sc, h.dtau_prev), h.bch, x);
                 x += res_words(plans[wave[m]]);
             }
-            if (!res_launch(ctx, bz, L, threads, smem)) {
-                if (first) return false;
-                throw ht3d_error(HT3D_ERR_CUDA, "cooperative launch refused between the waves of an ensemble");
-            }
-            first = false;
+            res_launch(ctx, bz, L, threads, smem);
             left.swap(rest);
         }
-        return true;
     };
 
     const int refresh_every = ctx->mixed_refresh;
@@ -1818,12 +1811,8 @@ void ht3d_ensemble_solve_mixed(ht3d_ctx* ctx, EnsSolveInst* in, int n) {
             while (resident && res_end < nitmax && !is_fp64(res_end + 1) && !is_storef(res_end + 1)) ++res_end;
             bool steady = res_end > iter && !storef;
             for (int q = 0; q < n && steady; ++q) steady = !H[q].active || H[q].dtau_prev == H[q].sc.dtau;
-            if (steady && !run_resident(iter, res_end, parity, prev0)) {  // one launch per iteration from here on
-                ctx->res_off = true;
-                resident = false;
-                steady = false;
-            }
             if (steady) {
+                run_resident(iter, res_end, parity, prev0);
                 window = res_end - iter + 1;
                 timer.count(window);
             } else {

@@ -522,19 +522,29 @@ inline ResPlan res_plan_full(const Pad& P, int sms) {
 inline int res_shortest(const ResPlan& r) { return r.bz == 5 ? 6 : 4; }
 inline size_t res_words(const ResPlan& r) { return (size_t)r.ctas() * 8 * res_faces(r.bz, r.nq, r.T); }
 
-// Face words of a launch: numbers of earlier iterations may stand in them, so
-// they are cleared only when they are allocated and when the numbers run out.
-inline u64* res_exchange(ht3d_ctx* ctx, size_t words, int iters, unsigned& tag) {
-    const size_t bytes = words * sizeof(u64);
-    const bool fresh = ctx->slot_bytes[SLOT_RES] < bytes;
-    u64* x = (u64*)ht3d_scratch(ctx, SLOT_RES, bytes);
-    if (fresh || ctx->res_tag > 0xffffffffu - (unsigned)iters - 1u) {
-        HT3D_CUDA(cudaMemsetAsync(x, 0, ctx->slot_bytes[SLOT_RES], ctx->stream));
+// Room for the face words of a launch; false where the device has none.  Numbers
+// of earlier iterations may stand in them, so they are cleared only when they are
+// allocated and when the numbers run out.
+inline bool res_reserve(ht3d_ctx* ctx, size_t words) {
+    if (ctx->slot_bytes[SLOT_RES] >= words * sizeof(u64)) return true;
+    try {
+        ht3d_scratch(ctx, SLOT_RES, words * sizeof(u64));
+    } catch (const ht3d_error& e) {
+        if (e.code != HT3D_ERR_NOMEM) throw;
+        return false;
+    }
+    HT3D_CUDA(cudaMemsetAsync(ctx->slot_ptr[SLOT_RES], 0, ctx->slot_bytes[SLOT_RES], ctx->stream));
+    ctx->res_tag = 0;
+    return true;
+}
+inline u64* res_exchange(ht3d_ctx* ctx, int iters, unsigned& tag) {
+    if (ctx->res_tag > 0xffffffffu - (unsigned)iters - 1u) {
+        HT3D_CUDA(cudaMemsetAsync(ctx->slot_ptr[SLOT_RES], 0, ctx->slot_bytes[SLOT_RES], ctx->stream));
         ctx->res_tag = 0;
     }
     tag = ctx->res_tag;
     ctx->res_tag += (unsigned)iters;
-    return x;
+    return (u64*)ctx->slot_ptr[SLOT_RES];
 }
 
 inline ResMember res_member(const ResPlan& r, const Pad& P, const float* D, const float* Dp, const float* Rin,
@@ -545,23 +555,32 @@ inline ResMember res_member(const ResPlan& r, const Pad& P, const float* D, cons
     return m;
 }
 
-// Launches the run; false when the device does not take the grid at once (the
-// caller then iterates one launch at a time).
-inline bool res_launch(ht3d_ctx* ctx, int bz, const ResLaunch& L, int threads, size_t smem) {
+inline const void* res_kernel(int bz) {
     static void (*const kern[])(ResLaunch) = {k_mixed_resident<1>, k_mixed_resident<2>, k_mixed_resident<3>,
                                               k_mixed_resident<5>, k_mixed_resident<7>};
-    const void* f = nullptr;
     for (size_t c = 0; c < std::size(kResBZ); ++c)
-        if (kResBZ[c] == bz) f = (const void*)kern[c];
+        if (kResBZ[c] == bz) return (const void*)kern[c];
+    throw ht3d_error(HT3D_ERR_ARG, "no kernel for columns of this height");
+}
+// Whether the device holds `blocks` CTAs of columns of bz planes at once (asked
+// when a run is planned: a launch that it then refuses is an error).
+inline bool res_fits(ht3d_ctx* ctx, int bz, int threads, size_t smem, long long blocks) {
+    const void* f = res_kernel(bz);
+    int coop = 0, optin = 0, per_sm = 0;
+    HT3D_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
+    HT3D_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    if (!coop || (size_t)optin < kResSmem) return false;
+    HT3D_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmem));
+    HT3D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, (threads + 31) / 32 * 32, smem));
+    return blocks <= (long long)per_sm * ctx->num_sms;
+}
+inline bool res_fits(ht3d_ctx* ctx, const ResPlan& r) {
+    return r.bz > 0 && res_fits(ctx, r.bz, r.T, res_smem(r.bz, r.nq, r.by), r.ctas());
+}
+
+inline void res_launch(ht3d_ctx* ctx, int bz, const ResLaunch& L, int threads, size_t smem) {
     void* args[] = {(void*)&L};
-    cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmem);
-    if (e == cudaSuccess)
-        e = cudaLaunchCooperativeKernel(f, dim3((unsigned)L.block0[L.n]), dim3((unsigned)((threads + 31) / 32 * 32)), args,
-                                        smem, ctx->stream);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
+    HT3D_CUDA(cudaLaunchCooperativeKernel(res_kernel(bz), dim3((unsigned)L.block0[L.n]),
+                                          dim3((unsigned)((threads + 31) / 32 * 32)), args, smem, ctx->stream));
     ctx->launches++;
-    return true;
 }

@@ -65,7 +65,6 @@ struct ht3d_ctx {
     void* h_ens = nullptr;                // pinned staging (instance records, results)
     size_t h_ens_bytes = 0;
     unsigned res_tag = 0;                 // iterations numbered so far by the resident kernel (this context)
-    bool res_off = false;                 // the device refused a cooperative launch: iterate one launch at a time
     int num_sms = 152;
     struct Room { const void* kern; int threads, most, fixed; };
     std::vector<Room> rooms;              // kernels asked for by even_smem: blocks per SM, static shared memory
