@@ -1234,18 +1234,16 @@ int ht3d_dyrel_solve_mixed(ht3d_ctx* ctx, double* X, const double* R, const doub
         derr = (int*)ht3d_scratch(ctx, SLOT_AUX0, sizeof(int) * 16);
         HT3D_CUDA(cudaMemsetAsync(derr, 0, sizeof(int), ctx->stream));
     }
-    // the run iter .. run_end (at least two iterations) in one launch
+    // the run iter .. run_end (res_shortest iterations at least) in one launch
     auto run_resident = [&](int iter, int run_end, const MixScal& s32, bool prev0, int cur, int prv) {
         ResLaunch L;
         L.n = 1;
         L.iters = run_end - iter + 1;
         L.prev0 = prev0 ? 1 : 0;
-        L.skip = ctx->wait_test;
-        L.limit = ctx->wait_test > 0 ? 1u << 12 : kResWaitLimit;
-        ctx->wait_test = 0;
         L.err = derr;
         L.block0[0] = 0;
         L.block0[1] = plan.ctas();
+        res_wait(ctx, L);
         u64* x = res_exchange(ctx, L.iters, L.tag);
         L.rec[0] = res_member(plan, P, Dbuf[cur], Dbuf[prv], Rin, kx32, ky32, kz32, Dbuf[cur], Dbuf[prv], s32, bch, x);
         res_launch(ctx, plan.bz, L, plan.T, res_smem(plan.bz, plan.nq, plan.by));
@@ -1721,8 +1719,6 @@ void ht3d_ensemble_solve_mixed(ht3d_ctx* ctx, EnsSolveInst* in, int n) {
             L.n = 0;
             L.iters = iters;
             L.prev0 = prev0;
-            L.skip = 0;
-            L.limit = kResWaitLimit;
             L.err = derr;
             L.block0[0] = 0;
             const int bz = plans[left[0]].bz, cap = ctx->num_sms;
@@ -1741,6 +1737,7 @@ void ht3d_ensemble_solve_mixed(ht3d_ctx* ctx, EnsSolveInst* in, int n) {
                 smem = std::max(smem, res_smem(p.bz, p.nq, p.by));
                 threads = std::max(threads, p.T);
             }
+            res_wait(ctx, L);
             u64* x = res_exchange(ctx, iters, L.tag);
             for (int m = 0; m < L.n; ++m) {
                 EnsHost& h = H[wave[m]];

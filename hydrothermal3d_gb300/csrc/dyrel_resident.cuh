@@ -123,7 +123,7 @@ struct ResLaunch {
     int n, iters, prev0;
     unsigned tag;  // iteration it publishes tag + it + 1
     unsigned limit;
-    int skip;      // test hook: CTA skip - 1 does not publish its faces
+    int skip;      // test hook: CTA skip - 1 of the launch does not publish its faces
     int* err;
     int block0[kResMaxPerLaunch + 1];
     ResMember rec[kResMaxPerLaunch];
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mixed_resident(const __grid_
     const u64 mom = pk(e.s.mom, e.s.mom), ndh2 = pk(-e.s.dh2, -e.s.dh2), cX = pk(e.s.cX, e.s.cX),
               dx2 = pk(_dx2f, _dx2f), dy2 = pk(_dy2f, _dy2f), dz2 = pk(_dz2f, _dz2f);
     const float* const Rcol = e.Rin + col;
-    const bool mute = L.skip == cta + 1, pubY = yedge && !mute, pubB = back && !mute, pubF = front && !mute;
+    const bool mute = L.skip == (int)blockIdx.x + 1, pubY = yedge && !mute, pubB = back && !mute, pubF = front && !mute;
     u64* const xch = e.xch;
     const unsigned hY = south ? hS : hN;
     // the neighbour blocks' cells next to this column: planes before and after
@@ -553,6 +553,20 @@ inline ResMember res_member(const ResPlan& r, const Pad& P, const float* D, cons
     ResMember m{D, Dp, Rin, kx, ky, kz, Dout, Dpout, xch, P, s, 0, r.nq, r.by, r.nby, r.T};
     for (int f = 0; f < 6; ++f) m.dir |= bc.dir[f] ? 1 << f : 0;
     return m;
+}
+
+// The launch's limit of polls and, for HT3D_TUNE_WAIT_TEST, the CTA that stays
+// silent; a launch in which no other CTA waits for that one leaves the test armed.
+inline void res_wait(ht3d_ctx* ctx, ResLaunch& L) {
+    L.skip = 0;
+    L.limit = kResWaitLimit;
+    const int v = ctx->wait_test;
+    for (int m = 0; m < L.n; ++m)
+        if (v > L.block0[m] && v <= L.block0[m + 1] && L.block0[m + 1] - L.block0[m] > 1) {
+            L.skip = v;
+            L.limit = 1u << 12;
+            ctx->wait_test = 0;
+        }
 }
 
 inline const void* res_kernel(int bz) {

@@ -88,11 +88,14 @@ extern "C" {
                                        per thread = 64x1, 128x1, 256x1, 64x8 (z-march),
                                        128x8, 128x16; overrides HT3D_TUNE_ENS_BLOCK;
                                        bit-identical results                             */
-#define HT3D_TUNE_WAIT_TEST 7       /* test hook of the bounded waits: v > 0 makes the next
-                                       two-iteration pass (HT3D_TUNE_TEMPORAL) skip the
-                                       copies of plane v - 1 and give up after 4096 polls;
-                                       the solve returns HT3D_ERR_TIMEOUT and the context
-                                       stays usable.  Reset after that pass.             */
+#define HT3D_TUNE_WAIT_TEST 7       /* test hook of the bounded waits, v > 0: the next
+                                       two-iteration pass (HT3D_TUNE_TEMPORAL) skips the
+                                       copies of plane v - 1, or the next resident run
+                                       whose block v - 1 (of all members' blocks) has
+                                       neighbours leaves that one silent; the waits give
+                                       up after 4096 polls, the solve (every member of an
+                                       ensemble) returns HT3D_ERR_TIMEOUT and the context
+                                       stays usable.  Reset by that pass or run.         */
 
 typedef struct ht3d_ctx ht3d_ctx;
 
