@@ -1686,6 +1686,10 @@ void ht3d_ensemble_solve_mixed(ht3d_ctx* ctx, EnsSolveInst* in, int n) {
         }
     bool graphs = ctx->ens_graphs != 0;
 
+    const int refresh_every = ctx->mixed_refresh;
+    auto is_fp64 = [&](int it) { return is_check(it, nitout) || (refresh_every > 0 && it % refresh_every == 0); };
+    auto is_storef = [&](int it) { return !is_fp64(it) && (it == nitmax || is_check(it + 1, nitout)); };
+
     // ---- runs of inner iterations in one launch per wave of members that fit
     // the chip together (unless the caller chose a tile shape)
     std::vector<ResPlan> plans(n);
@@ -1696,7 +1700,62 @@ void ht3d_ensemble_solve_mixed(ht3d_ctx* ctx, EnsSolveInst* in, int n) {
         resident = resident && res_fits(ctx, plans[q]);
         cta_words = std::max(cta_words, resident ? res_words(plans[q]) / plans[q].ctas() : 0);
     }
-    resident = resident && res_reserve(ctx, cta_words * ctx->num_sms);
+    // the active members in waves: equal columns together, the largest grids
+    // first, then whatever still fits
+    auto active_waves = [&]() {
+        std::vector<int> left;
+        for (int q : order)
+            if (H[q].active) left.push_back(q);
+        std::stable_sort(left.begin(), left.end(), [&](int a, int b) {
+            return plans[a].bz != plans[b].bz ? plans[a].bz > plans[b].bz : plans[a].ctas() > plans[b].ctas();
+        });
+        std::vector<std::vector<int>> waves;
+        while (!left.empty()) {
+            std::vector<int> wave, rest;
+            int blocks = 0;
+            for (int q : left) {
+                const ResPlan& p = plans[q];
+                if (p.bz != plans[left[0]].bz || (int)wave.size() == kResMaxPerLaunch || blocks + p.ctas() > ctx->num_sms) {
+                    rest.push_back(q);
+                    continue;
+                }
+                wave.push_back(q);
+                blocks += p.ctas();
+            }
+            waves.push_back(wave);
+            left.swap(rest);
+        }
+        return waves;
+    };
+    // Whether runs of that many iterations pay.  Each wave loads and stores its members
+    // once and takes a column's time per iteration; the batched kernel takes what memory
+    // needs for the cells of all of them (28 B each, from L2 for the first 4 million),
+    // with replayed windows less per launch but 150 us for their capture, once a check.
+    // Fitted to steps of ensembles of 1 to 64 members, 16^3 to 111 x 97 x 113, checks
+    // every 4 to 600 iterations; runs of k iterations, ms a step in one launch a wave
+    // and batched: 32 x 95^3, k = 2, 174 and 154, k = 508 within 1 %; 16 x 79^3, k = 2,
+    // 61.2 and 57.4, k = 10, 29.5 and 30.8; 63^3 alone, k = 2, 5.28 and 4.95, k = 28 half
+    // the batched time, k = 508 a tenth more; 64 of 31 to 95 cells a side, k = 2 5 %
+    // more, k = 28 a fifth less, k = 508 a third less.
+    auto run_pays = [&](int iters) {
+        const auto waves = active_waves();
+        double res = 0.0, cells = 0.0;  // us
+        for (const auto& wave : waves) {
+            double c = 0.0, t = 0.0;
+            for (int q : wave) {
+                c += (double)H[q].P.size;
+                t = std::max(t, res_time(plans[q], H[q].P));
+            }
+            res += 4.0 + 8.5e-6 * c + iters * t;
+            cells += c;
+        }
+        const bool replay = graphs && iters > kEnsGraphIters;
+        const double beyond = std::max(0.0, cells - 4e6);
+        return res < (replay ? 150.0 + iters * (2.4 + 3.6e-6 * cells + 0.7e-6 * beyond) : iters * (3.3 + 4.6e-6 * cells));
+    };
+    // (asked once for the solve, of a run between two checks or refreshes)
+    const int longest = std::min({nitmax, nitout, refresh_every > 0 ? refresh_every : nitmax}) - 2;
+    resident = resident && longest > 1 && run_pays(longest) && res_reserve(ctx, cta_words * ctx->num_sms);
     int* derr = nullptr;
     if (resident) {
         tuning = false;
@@ -1707,31 +1766,17 @@ void ht3d_ensemble_solve_mixed(ht3d_ctx* ctx, EnsSolveInst* in, int n) {
     // iterations iter .. res_end of every active member, a wave after the other
     auto run_resident = [&](int iter, int res_end, int parity, int prev0) {
         const int iters = res_end - iter + 1, to = (parity + iters) & 1;
-        std::vector<int> left;
-        for (int q : order)
-            if (H[q].active) left.push_back(q);
-        // equal columns together, the largest grids first, then whatever still fits
-        std::stable_sort(left.begin(), left.end(), [&](int a, int b) {
-            return plans[a].bz != plans[b].bz ? plans[a].bz > plans[b].bz : plans[a].ctas() > plans[b].ctas();
-        });
-        while (!left.empty()) {
+        for (const std::vector<int>& wave : active_waves()) {
             ResLaunch L;
             L.n = 0;
             L.iters = iters;
             L.prev0 = prev0;
             L.err = derr;
             L.block0[0] = 0;
-            const int bz = plans[left[0]].bz, cap = ctx->num_sms;
-            std::vector<int> wave, rest;
             size_t smem = 0;
             int threads = 0;
-            for (int q : left) {
+            for (int q : wave) {
                 const ResPlan& p = plans[q];
-                if (p.bz != bz || L.n == kResMaxPerLaunch || L.block0[L.n] + p.ctas() > cap) {
-                    rest.push_back(q);
-                    continue;
-                }
-                wave.push_back(q);
                 L.block0[L.n + 1] = L.block0[L.n] + p.ctas();
                 ++L.n;
                 smem = std::max(smem, res_smem(p.bz, p.nq, p.by));
@@ -1745,14 +1790,10 @@ void ht3d_ensemble_solve_mixed(ht3d_ctx* ctx, EnsSolveInst* in, int n) {
                                       h.f32[6], h.f32[to], h.f32[to ^ 1], mix_scal(h.sc, h.dtau_prev), h.bch, x);
                 x += res_words(plans[wave[m]]);
             }
-            res_launch(ctx, bz, L, threads, smem);
-            left.swap(rest);
+            res_launch(ctx, plans[wave[0]].bz, L, threads, smem);
         }
     };
 
-    const int refresh_every = ctx->mixed_refresh;
-    auto is_fp64 = [&](int it) { return is_check(it, nitout) || (refresh_every > 0 && it % refresh_every == 0); };
-    auto is_storef = [&](int it) { return !is_fp64(it) && (it == nitmax || is_check(it + 1, nitout)); };
     InnerTimer timer(ctx);
     int nactive = nused;
     int prev0 = 1;  // the previous corrections are 0 (start, or D just folded): same for every member

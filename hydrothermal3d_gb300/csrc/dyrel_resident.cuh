@@ -520,6 +520,11 @@ inline ResPlan res_plan_full(const Pad& P, int sms) {
 // 131 15.9 and 15.7; of four 2.32 and 2.31, 6.83 and 6.46, 11.4 and 11.6; of six 1.79
 // and 1.89, 5.29 and 5.33, 9.09 and 9.35.
 inline int res_shortest(const ResPlan& r) { return r.bz == 5 ? 6 : 4; }
+// us per iteration of a wave whose tallest plan this is (within a tenth or so of
+// the figures above and of 31^3 to 127^3, thin and long grids as ensembles)
+inline double res_time(const ResPlan& r, const Pad& P) {
+    return 1.2 + 0.00095 * r.T * std::min(r.bz, P.nz) + (r.nby > 1 ? 0.0009 * r.bz * r.nq : 0.0);
+}
 inline size_t res_words(const ResPlan& r) { return (size_t)r.ctas() * 8 * res_faces(r.bz, r.nq, r.T); }
 
 // Room for the face words of a launch; false where the device has none.  Numbers
