@@ -1,6 +1,6 @@
 // Plain FP64 DYREL solver.  Compiled with -fmad=false: every pseudo-iteration
-// rounds exactly like the reference's separate kernels (no FMA contraction,
-// F divided by PC), so the solver differs from the reference only through the
+// rounds like the reference's separate kernels (no FMA contraction, F's quotient
+// by PC as fp64_div.cuh says), so the solver differs from the reference only through the
 // summation order of its norm and Rayleigh-quotient reductions.
 #include "dyrel_f64.cuh"
 

@@ -70,7 +70,8 @@ extern "C" {
                                        FP32 inner-iteration launches with CUDA events on the
                                        ctx stream (read back by ht3d_ctx_inner_timing)    */
 #define HT3D_TUNE_ENS_BLOCK 4       /* threads per block of the batched ensemble iteration
-                                       with one plane per thread: 64/128/256 fixes it, 0
+                                       with one plane per thread: 64/128/256 fixes it and
+                                       turns resident runs off (HT3D_TUNE_TEMPORAL), 0
                                        leaves the tile shape to HT3D_TUNE_ENS_TILE        */
 #define HT3D_TUNE_ENS_GRAPH 5       /* 1 (default): replay windows of 16 batched inner
                                        iterations as CUDA graphs; 0: launch one by one    */
@@ -81,10 +82,16 @@ extern "C" {
                                        tiles to >= 3/4, one per launch otherwise; >= 2 = two
                                        per pass on every grid, that many planes per chunk;
                                        bit-identical results (255^3: 59.6 against 75.8 us
-                                       per iteration)                                    */
+                                       per iteration).  1 also keeps runs of iterations of
+                                       grids that fit the chip, and of ensembles of such
+                                       grids, in one launch (resident runs); any other
+                                       value turns these off                             */
 #define HT3D_TUNE_ENS_TILE 8        /* tile shape of the batched ensemble iteration: 0 =
-                                       autotune on first use of an ensemble shape over
-                                       six shapes, or 1..6 fixed: threads per block x planes
+                                       resident runs where every member fits the chip and
+                                       they pay (other iterations 128x1), else autotune on
+                                       first use of an ensemble shape over six shapes; 1..6
+                                       fixed, without resident runs (of single solves of
+                                       this context too): threads per block x planes
                                        per thread = 64x1, 128x1, 256x1, 64x8 (z-march),
                                        128x8, 128x16; overrides HT3D_TUNE_ENS_BLOCK;
                                        bit-identical results                             */
