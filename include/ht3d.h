@@ -98,11 +98,11 @@ extern "C" {
 #define HT3D_TUNE_WAIT_TEST 7       /* test hook of the bounded waits, v > 0: the next
                                        two-iteration pass (HT3D_TUNE_TEMPORAL) skips the
                                        copies of plane v - 1, or the next resident run
-                                       whose block v - 1 (of all members' blocks) has
-                                       neighbours leaves that one silent; the waits give
-                                       up after 4096 polls, the solve (every member of an
-                                       ensemble) returns HT3D_ERR_TIMEOUT and the context
-                                       stays usable.  Reset by that pass or run.         */
+                                       with a block v - 1 that has neighbours (in any
+                                       member of an ensemble) leaves it silent; the waits
+                                       give up after 4096 polls, the solve (every member)
+                                       returns HT3D_ERR_TIMEOUT and the context stays
+                                       usable.  Reset by that pass or run.               */
 
 typedef struct ht3d_ctx ht3d_ctx;
 
